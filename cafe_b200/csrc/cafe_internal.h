@@ -5,6 +5,8 @@
 
 #include "cafe_types.h"
 
+struct CafeSortDesc;   // radix_sort.cuh
+
 
 #define CAFE_MAX_DIM 128      // widest embedding row the scatter workspace is sized for
 #define CAFE_CHUNK 32         // sorted lookups reduced by one thread group in the scatter
@@ -22,17 +24,14 @@ struct CafeEmbedWorkspace {
     float* totals = nullptr;     // [CAFE_MAX_SEGMENTS] sum of norms per field
     int32_t* mask = nullptr;     // [cap] newly-hot flag per lookup
     int32_t* post_row = nullptr; // [cap] hot row after the lookup's own call
-    uint32_t* key[2] = {nullptr, nullptr};   // [cap] unified row key, unsorted / sorted
-    int32_t* pos[2] = {nullptr, nullptr};    // [cap] lookup position: intermediate pass of the sort / sorted
+    uint32_t* key = nullptr;                 // [cap] unified row key of every lookup
+    uint2* rows = nullptr;                   // [cap] (row key, position) sorted by row
     float* partial = nullptr;    // [2 * ceil(cap/CAFE_CHUNK) * CAFE_MAX_DIM] partial row sums of chunk-spanning rows
     int32_t* row_winner = nullptr;   // [hotn] migration: highest position that claims a hot row in this call (-1 between calls)
-    uint32_t* key_tmp = nullptr;     // [cap] intermediate keys of the row sort
-    uint32_t* bucket_key[2] = {nullptr, nullptr};   // [cap] main / LRU bucket of every lookup, left by cafe_embed_resolve ...
-    const uint32_t* keys_of = nullptr;              // ... for the lookups whose global ids are in this array
+    uint2* rows_tmp = nullptr;       // [cap] pairs between two passes of the row sort
+    const uint32_t* keys_of = nullptr;   // `key` was left by cafe_embed_resolve for the lookups whose global ids are in this array
     int keys_total = 0;
     int32_t* sort_scratch = nullptr; // radix-sort histograms
-    cudaStream_t side = nullptr;     // runs the scatter's key sort beside the sketch insert
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t late = nullptr;     // importance of fields whose gradients arrive behind a gate
     cudaEvent_t ev_late = nullptr;
     // arrays whose side work cafe_embed_backward_begin has already started (null: none)
@@ -49,8 +48,12 @@ CafeEmbedWorkspace* cafe_internal_ws(void* h);
 int cafe_internal_insert(void* h, const uint32_t* gid, const float* imp, const int* seg_off, int nseg, int32_t* mask,
                          int32_t* post_row, int mode, cudaStream_t stream);
 // starts the insert's bucket sorts of `gid` beside whatever the caller queues next on `stream`
-// (key1 / key2: the lookups' main / LRU bucket numbers if the caller has them, else null)
-void cafe_internal_presort(void* h, const uint32_t* gid, int n, const uint32_t* key1, const uint32_t* key2, cudaStream_t stream);
+// (also: a further sort to run with them, or null).  A null gid withdraws an earlier presort.
+void cafe_internal_presort(void* h, const uint32_t* gid, int n, const CafeSortDesc* also, cudaStream_t stream);
+// makes `stream` wait for sorts that a presort started: before their inputs are written again (they stay outstanding for
+// the call that uses them), or to use them
+int cafe_internal_sort_wait(void* h, cudaStream_t stream);
+int cafe_internal_sort_join(void* h, cudaStream_t stream);
 // counts of segments >= seg of the next cafe_internal_insert are valid once `ev` has fired (null: no gate)
 void cafe_internal_set_gate(void* h, int seg, cudaEvent_t ev);
 void cafe_internal_set_error(const char* msg);

@@ -51,7 +51,7 @@ __device__ __forceinline__ T* shfl_ptr(T* p, int src) {
 template <int G, typename IdT>
 __global__ void __launch_bounds__(256)
 k_embed_forward(const __grid_constant__ CafeFields F, const IdT* __restrict__ ids,
-                const CafeMainBucket* __restrict__ mb, int n1, const CafeRankBuffers out, int64_t field_stride,
+                const CafeMainBucket* __restrict__ mb, const CafeMod n1, const CafeRankBuffers out, int64_t field_stride,
                 int64_t sample_stride, uint32_t* __restrict__ gid_out, int32_t* __restrict__ row_out, int total) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -98,21 +98,25 @@ k_embed_forward(const __grid_constant__ CafeFields F, const IdT* __restrict__ id
     }
 }
 
-// The forward in two kernels, for training: k_embed_resolve does the sketch probe only (global id, row code,
-// and the two bucket numbers the insert will sort by), k_embed_gather copies the rows named by the codes.
+// unified row number of a row code: hot rows first, then every field's hash rows
+__device__ __forceinline__ uint32_t cafe_row_key(const CafeFields& F, int32_t code, int f) {
+    return code < 0 ? (uint32_t)((-code) % F.hotn) : (uint32_t)(F.hotn + F.hash_base[f] + code);
+}
+
+// The forward in two kernels, for training: k_embed_resolve does the sketch probe only (global id, row code, and the
+// unified row that the backward sorts by), k_embed_gather copies the rows named by the codes.
 // Between the two the caller can start the backward's sorts, which need nothing but the first kernel's
 // outputs, so that they run beside the gather instead of after it.
 template <typename IdT>
 __global__ void __launch_bounds__(256)
 k_embed_resolve(const __grid_constant__ CafeFields F, const IdT* __restrict__ ids, const CafeMainBucket* __restrict__ mb,
-                int n1, int n2, uint32_t* __restrict__ gid_out, int32_t* __restrict__ row_out, uint32_t* __restrict__ key1_out,
-                uint32_t* __restrict__ key2_out, int total) {
+                const CafeMod n1, uint32_t* __restrict__ gid_out, int32_t* __restrict__ row_out, uint32_t* __restrict__ rowkey_out,
+                int total) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= total) return;
     const int f = p / F.B;
     const uint32_t x = (uint32_t)((int64_t)ids[p] + (int64_t)F.f_offset[f]);
-    const int32_t k1 = cafe_hash(x, n1);
-    const CafeMainBucket* bk = &mb[k1];
+    const CafeMainBucket* bk = &mb[cafe_hash(x, n1)];
     const uint4 v = *reinterpret_cast<const uint4*>(bk->val);
     const int4 d = *reinterpret_cast<const int4*>(bk->dic);
     int32_t r = 0;
@@ -121,8 +125,9 @@ k_embed_resolve(const __grid_constant__ CafeFields F, const IdT* __restrict__ id
     if (v.y == x && d.y != 0) r = d.y;
     if (v.x == x && d.x != 0) r = d.x;
     gid_out[p] = x;
-    row_out[p] = r ? -r : (int32_t)(x % (uint32_t)F.hash_size[f]);
-    if (key1_out) { key1_out[p] = (uint32_t)k1; key2_out[p] = (uint32_t)cafe_hash(x, n2); }
+    const int32_t code = r ? -r : (int32_t)(x % (uint32_t)F.hash_size[f]);
+    row_out[p] = code;
+    if (rowkey_out) rowkey_out[p] = cafe_row_key(F, code, f);
 }
 
 template <int G>
@@ -276,8 +281,7 @@ __global__ void k_row_keys(const __grid_constant__ CafeFields F, const int32_t* 
                            uint32_t* __restrict__ key) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= total) return;
-    const int32_t r = row[p];
-    key[p] = r < 0 ? (uint32_t)((-r) % F.hotn) : (uint32_t)(F.hotn + F.hash_base[p / F.B] + r);
+    key[p] = cafe_row_key(F, row[p], p / F.B);
 }
 
 __device__ __forceinline__ float* row_ptr(const CafeFields& F, uint32_t key, int pos) {
@@ -298,8 +302,7 @@ __device__ __forceinline__ void sgd_apply(float* w, float4 g, float lr) {
 template <int G>
 __global__ void __launch_bounds__(256, 4)
 k_scatter_chunks(const __grid_constant__ CafeFields F, const float* __restrict__ grad, int64_t field_stride,
-                 int64_t sample_stride, const uint32_t* __restrict__ skey, const int32_t* __restrict__ spos, int M,
-                 float lr, float* __restrict__ partial) {
+                 int64_t sample_stride, const uint2* __restrict__ rows, int M, float lr, float* __restrict__ partial) {
     constexpr int PER = CAFE_CHUNK / G;   // sorted entries held per lane
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t chunk = t / G;
@@ -312,11 +315,12 @@ k_scatter_chunks(const __grid_constant__ CafeFields F, const float* __restrict__
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int j = i * G + gl;
-        k[i] = j < cnt ? skey[base + j] : NOKEY;
-        q[i] = j < cnt ? spos[base + j] : 0;
+        const uint2 e = j < cnt ? rows[base + j] : make_uint2(NOKEY, 0u);
+        k[i] = e.x;
+        q[i] = (int32_t)e.y;
     }
-    const uint32_t key_prev = (cnt > 0 && base > 0) ? skey[base - 1] : NOKEY;
-    const uint32_t key_next = (cnt > 0 && base + CAFE_CHUNK < M) ? skey[base + CAFE_CHUNK] : NOKEY;
+    const uint32_t key_prev = (cnt > 0 && base > 0) ? rows[base - 1].x : NOKEY;
+    const uint32_t key_next = (cnt > 0 && base + CAFE_CHUNK < M) ? rows[base + CAFE_CHUNK].x : NOKEY;
 
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t cur = NOKEY;
@@ -370,22 +374,22 @@ k_scatter_chunks(const __grid_constant__ CafeFields F, const float* __restrict__
 // One group per chunk; the chunk in which a spanning row STARTS adds up that row's partial sums.
 template <int G>
 __global__ void __launch_bounds__(256)
-k_scatter_fixup(const __grid_constant__ CafeFields F, const uint32_t* __restrict__ skey,
-                const int32_t* __restrict__ spos, int M, float lr, const float* __restrict__ partial) {
+k_scatter_fixup(const __grid_constant__ CafeFields F, const uint2* __restrict__ rows, int M, float lr, const float* __restrict__ partial) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t chunk = t / G;
     const int c = (int)(t % G) * 4;
     const int64_t base = chunk * CAFE_CHUNK;
     if (base + CAFE_CHUNK >= M) return;   // the last chunk cannot continue to the right
-    const uint32_t key = skey[base + CAFE_CHUNK - 1];
-    if (key != skey[base + CAFE_CHUNK]) return;            // its last row ends with the chunk
-    const bool single = skey[base] == key;
-    if (single && base > 0 && skey[base - 1] == key) return;   // the row started in an earlier chunk
+    const uint2 last = rows[base + CAFE_CHUNK - 1];
+    const uint32_t key = last.x;
+    if (key != rows[base + CAFE_CHUNK].x) return;            // its last row ends with the chunk
+    const bool single = rows[base].x == key;
+    if (single && base > 0 && rows[base - 1].x == key) return;   // the row started in an earlier chunk
     // end of the row's range in the sorted keys
     int64_t lo = base + CAFE_CHUNK, hi = M;   // first index with key' > key lies in (lo, hi]
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
-        if (skey[mid] <= key) lo = mid + 1; else hi = mid;
+        if (rows[mid].x <= key) lo = mid + 1; else hi = mid;
     }
     const int64_t last_chunk = (lo - 1) / CAFE_CHUNK;
     float4 acc = *reinterpret_cast<const float4*>(partial + (size_t)(chunk * 2 + (single ? 0 : 1)) * CAFE_MAX_DIM + c);
@@ -399,7 +403,7 @@ k_scatter_fixup(const __grid_constant__ CafeFields F, const uint32_t* __restrict
         for (int u = 0; u < U; ++u)
             if (c0 + u <= last_chunk) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
     }
-    sgd_apply(row_ptr(F, key, spos[base + CAFE_CHUNK - 1]) + c, acc, lr);
+    sgd_apply(row_ptr(F, key, (int)last.y) + c, acc, lr);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -595,16 +599,11 @@ int cafe_embed_ws_init(CafeEmbedWorkspace* ws, int cap, int hotn) {
     auto A = [&](void** p, size_t n) { if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1); };
     A((void**)&ws->norm, 4 * M); A((void**)&ws->imp, 4 * M); A((void**)&ws->totals, 4 * CAFE_MAX_SEGMENTS);
     A((void**)&ws->mask, 4 * M); A((void**)&ws->post_row, 4 * M);
-    for (int i = 0; i < 2; ++i) { A((void**)&ws->key[i], 4 * M); A((void**)&ws->pos[i], 4 * M); }
+    A((void**)&ws->key, 4 * M); A((void**)&ws->rows, sizeof(uint2) * M); A((void**)&ws->rows_tmp, sizeof(uint2) * M);
     A((void**)&ws->partial, sizeof(float) * 2 * chunks * CAFE_MAX_DIM);
     A((void**)&ws->row_winner, 4 * (size_t)(hotn > 0 ? hotn : 1));
     if (e == cudaSuccess) e = cudaMemset(ws->row_winner, 0xff, 4 * (size_t)(hotn > 0 ? hotn : 1));   // -1: unclaimed
-    A((void**)&ws->key_tmp, 4 * M);
-    A((void**)&ws->bucket_key[0], 4 * M); A((void**)&ws->bucket_key[1], 4 * M);
-    A((void**)&ws->sort_scratch, 4 * cafe_rs_scratch_elems(cap));
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws->side, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws->ev_fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws->ev_join, cudaEventDisableTiming);
+    A((void**)&ws->sort_scratch, 4 * cafe_rs_scratch_elems());
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws->late, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws->ev_late, cudaEventDisableTiming);
     if (e != cudaSuccess) { cafe_internal_set_error(cudaGetErrorString(e)); return CAFE_ERR_CUDA; }
@@ -612,12 +611,9 @@ int cafe_embed_ws_init(CafeEmbedWorkspace* ws, int cap, int hotn) {
 }
 
 void cafe_embed_ws_free(CafeEmbedWorkspace* ws) {
-    void* ptrs[] = {ws->norm, ws->imp, ws->totals, ws->mask, ws->post_row, ws->key[0], ws->key[1], ws->pos[0], ws->pos[1],
-                    ws->partial, ws->key_tmp, ws->sort_scratch, ws->row_winner, ws->bucket_key[0], ws->bucket_key[1]};
+    void* ptrs[] = {ws->norm, ws->imp, ws->totals, ws->mask, ws->post_row, ws->key, ws->rows,
+                    ws->rows_tmp, ws->partial, ws->sort_scratch, ws->row_winner};
     for (void* p : ptrs) if (p) cudaFree(p);
-    if (ws->side) { cudaStreamSynchronize(ws->side); cudaStreamDestroy(ws->side); }
-    if (ws->ev_fork) cudaEventDestroy(ws->ev_fork);
-    if (ws->ev_join) cudaEventDestroy(ws->ev_join);
     if (ws->late) { cudaStreamSynchronize(ws->late); cudaStreamDestroy(ws->late); }
     if (ws->ev_late) cudaEventDestroy(ws->ev_late);
     *ws = CafeEmbedWorkspace();
@@ -676,10 +672,10 @@ static int launch_forward(const CafeFields& F, const void* ids_dev, int ids_are_
     const int blocks = (warps + 7) / 8;
     CAFE_PROF(CAFE_P_FORWARD, st);
     if (ids_are_int64) {
-        DISPATCH_G(D, (k_embed_forward<G, int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, V.n1, out_dev,
+        DISPATCH_G(D, (k_embed_forward<G, int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, cafe_mod_of(V.n1), out_dev,
                        out_field_stride, out_sample_stride, gid_out_dev, row_out_dev, total)));
     } else {
-        DISPATCH_G(D, (k_embed_forward<G, int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, V.n1, out_dev,
+        DISPATCH_G(D, (k_embed_forward<G, int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, cafe_mod_of(V.n1), out_dev,
                        out_field_stride, out_sample_stride, gid_out_dev, row_out_dev, total)));
     }
     return fail_cuda("cafe_embed_forward");
@@ -735,25 +731,31 @@ int cafe_embed_resolve(void* h, const void* ids_dev, int ids_are_int64, int nfie
     CafeFields F;
     memset(&F, 0, sizeof(F));
     F.nfields = nfields; F.B = B; F.hotn = hotn;
+    int64_t rows = 0;
     for (int f = 0; f < nfields; ++f) {
         if (hash_size[f] < 1) return CAFE_ERR_ARG;
-        F.f_offset[f] = (uint32_t)f_offset[f]; F.hash_size[f] = hash_size[f];
+        F.f_offset[f] = (uint32_t)f_offset[f]; F.hash_size[f] = hash_size[f]; F.hash_base[f] = (int32_t)rows;
+        rows += hash_size[f];
     }
     CafeSketchView V = cafe_internal_view(h);
     if (hotn != V.lim) return CAFE_ERR_ARG;
     CafeEmbedWorkspace* ws = cafe_internal_ws(h);
     const int total = (int)total64;
-    // the bucket numbers are kept for the insert's sorts when the lookups fit the workspace
-    const bool keep = total <= ws->cap;
-    uint32_t* k1 = keep ? ws->bucket_key[0] : nullptr;
-    uint32_t* k2 = keep ? ws->bucket_key[1] : nullptr;
+    // the row keys are kept for the backward when the lookups fit the workspace (and rows fit the unified numbering)
+    const bool keep = total <= ws->cap && rows + hotn <= 0x7fffffffLL;
+    uint32_t* keys = keep ? ws->key : nullptr;
+    const CafeMod mod = cafe_mod_of(V.n1);
     ws->keys_of = keep ? gid_out_dev : nullptr;
     ws->keys_total = keep ? total : 0;
     cudaStream_t st = (cudaStream_t)stream;
+    if (keep) {   // sorts of an earlier forward may still be reading the keys
+        const int rc = cafe_internal_sort_wait(h, st);
+        if (rc != CAFE_OK) return rc;
+    }
     CAFE_PROF(CAFE_P_QUERY, st);
     const int blocks = (total + 255) / 256;
-    if (ids_are_int64) k_embed_resolve<int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, V.n1, V.n2, gid_out_dev, row_out_dev, k1, k2, total);
-    else k_embed_resolve<int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, V.n1, V.n2, gid_out_dev, row_out_dev, k1, k2, total);
+    if (ids_are_int64) k_embed_resolve<int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, keys, total);
+    else k_embed_resolve<int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, keys, total);
     return fail_cuda("cafe_embed_resolve");
 }
 
@@ -907,18 +909,25 @@ int cafe_migrate(void* h, const void* ids_dev, int ids_are_int64, const int32_t*
 // The scatter in two parts.  scatter_prepare needs only the forward's row numbers (unified row keys and
 // their radix sort); scatter_apply reads the sorted keys, the gradient and the tables.  The split lets a
 // caller run the first part on the workspace's side stream while the sketch insert runs on the main one.
-static int scatter_prepare(CafeEmbedWorkspace* ws, const CafeFields& F, const int32_t* row_dev, int total, int hotn,
-                           cudaStream_t st) {
-    { CAFE_PROF(CAFE_P_ROWKEYS, st); k_row_keys<<<(total + 255) / 256, 256, 0, st>>>(F, row_dev, total, ws->key[0]); }
-    int bits = 1;
-    while ((1ll << bits) < (int64_t)hotn + F.hash_base[F.nfields]) ++bits;
-    cudaError_t e;
-    { CAFE_PROF(CAFE_P_ROWSORT, st);
-      // (row key, position) pairs, stable: a row's lookups stay in batch order, which fixes the order of the additions
-      CafeKeySource src;
-      src.key = ws->key[0]; src.gid = nullptr; src.nb = 0;
-      e = cafe_radix_sort(src, nullptr, ws->key_tmp, ws->pos[0], ws->key[1], ws->pos[1], total, bits, ws->sort_scratch, nullptr,
-                          nullptr, st); }
+static CafeSortDesc row_sort_desc(CafeEmbedWorkspace* ws, const CafeFields& F, int total) {
+    // (row key, position) pairs, stable: a row's lookups stay in batch order, which fixes the order of the additions
+    CafeSortDesc D;
+    memset(&D, 0, sizeof(D));
+    D.in = ws->key; D.mod.n = F.hotn + F.hash_base[F.nfields]; D.n = total;
+    D.tmp = ws->rows_tmp; D.out = ws->rows; D.scratch = ws->sort_scratch;
+    return D;
+}
+static void row_keys(CafeEmbedWorkspace* ws, const CafeFields& F, const int32_t* row_dev, int total, cudaStream_t st) {
+    CAFE_PROF(CAFE_P_ROWKEYS, st);
+    k_row_keys<<<(total + 255) / 256, 256, 0, st>>>(F, row_dev, total, ws->key);
+}
+static int scatter_prepare(CafeEmbedWorkspace* ws, const CafeFields& F, const int32_t* row_dev, int total, cudaStream_t st) {
+    row_keys(ws, F, row_dev, total, st);
+    CAFE_PROF(CAFE_P_ROWSORT, st);
+    CafeSortBatch B;
+    B.count = 1;
+    B.d[0] = row_sort_desc(ws, F, total);
+    const cudaError_t e = cafe_radix_sort(B, st);
     if (e != cudaSuccess) { cafe_internal_set_error(cudaGetErrorString(e)); return CAFE_ERR_CUDA; }
     return CAFE_OK;
 }
@@ -928,9 +937,9 @@ static int scatter_apply(CafeEmbedWorkspace* ws, const CafeFields& F, const floa
     const int64_t chunks = ((int64_t)total + CAFE_CHUNK - 1) / CAFE_CHUNK;
     { CAFE_PROF(CAFE_P_SCATTER, st);
     DISPATCH_G(D, (k_scatter_chunks<G><<<(unsigned)((chunks * G + 255) / 256), 256, 0, st>>>(F, grad_dev, field_stride,
-                   sample_stride, ws->key[1], ws->pos[1], total, lr, ws->partial))); }
+                   sample_stride, ws->rows, total, lr, ws->partial))); }
     { CAFE_PROF(CAFE_P_FIXUP, st);
-    DISPATCH_G(D, (k_scatter_fixup<G><<<(unsigned)((chunks * G + 255) / 256), 256, 0, st>>>(F, ws->key[1], ws->pos[1], total,
+    DISPATCH_G(D, (k_scatter_fixup<G><<<(unsigned)((chunks * G + 255) / 256), 256, 0, st>>>(F, ws->rows, total,
                    lr, ws->partial))); }
     return fail_cuda("cafe_scatter_sgd");
 }
@@ -958,47 +967,31 @@ int cafe_scatter_sgd(void* h, const float* grad_dev, int64_t field_stride, int64
     if (total == 0) return CAFE_OK;
     CafeEmbedWorkspace* ws = cafe_internal_ws(h);
     cudaStream_t st = (cudaStream_t)stream;
-    rc = scatter_prepare(ws, F, row_dev, total, hotn, st);
+    // the row keys of an earlier cafe_embed_resolve and the row order of an earlier head start are overwritten
+    ws->keys_of = nullptr;
+    ws->begun_gid = nullptr;
+    rc = cafe_internal_sort_wait(h, st);
+    if (rc != CAFE_OK) return rc;
+    rc = scatter_prepare(ws, F, row_dev, total, st);
     if (rc != CAFE_OK) return rc;
     return scatter_apply(ws, F, grad_dev, field_stride, sample_stride, total, D, lr, st);
 }
 
-// Starts scatter_prepare on the side stream, ordered after everything already queued on `st`.
-static int scatter_prepare_aside(CafeEmbedWorkspace* ws, const CafeFields& F, const int32_t* row_dev, int total, int hotn,
-                                 cudaStream_t st) {
-    if (cafe_prof_serialise()) {
-        int rc0 = scatter_prepare(ws, F, row_dev, total, hotn, st);
-        cudaEventRecord(ws->ev_join, st);
-        return rc0;
-    }
-    if (cudaEventRecord(ws->ev_fork, st) != cudaSuccess || cudaStreamWaitEvent(ws->side, ws->ev_fork, 0) != cudaSuccess)
-        return fail_cuda("scatter fork");
-    int rc = scatter_prepare(ws, F, row_dev, total, hotn, ws->side);
-    // the join is recorded even after a failure so that the main stream never waits on a stale event
-    if (cudaEventRecord(ws->ev_join, ws->side) != cudaSuccess) return fail_cuda("scatter join");
-    return rc;
-}
-// Starts (or recognises as already started by cafe_embed_backward_begin) the side work of one backward
-// call: the scatter's row sort and, for the parallel insert, the sketch's bucket sorts.
+// Starts (or recognises as already started by cafe_embed_backward_begin) the side work of one backward call: the row sort
+// of the scatter and the bucket sorts of the parallel insert, in one batch on a stream of the sketch's.
 static int backward_side_work(void* h, CafeEmbedWorkspace* ws, const CafeFields& FS, const uint32_t* gid_dev,
-                              const int32_t* row_dev, int total, int hotn, int insert_mode, cudaStream_t st) {
+                              const int32_t* row_dev, int total, int insert_mode, cudaStream_t st) {
     const bool begun = ws->begun_gid == gid_dev && ws->begun_row == row_dev && ws->begun_total == total &&
                        ws->begun_mode == insert_mode && gid_dev != nullptr;
     ws->begun_gid = nullptr; ws->begun_row = nullptr; ws->begun_total = 0;
     if (begun) return CAFE_OK;
-    // the sketch's two sorts are queued first (the insert needs them long before the scatter needs the row sort) ...
-    if (insert_mode != CAFE_INSERT_SEQUENTIAL) {
-        // bucket numbers left by cafe_embed_resolve for exactly these lookups save the sorts their hashing
-        const bool have = ws->keys_of == gid_dev && ws->keys_total == total;
-        cafe_internal_presort(h, gid_dev, total, have ? ws->bucket_key[0] : nullptr, have ? ws->bucket_key[1] : nullptr, st);
-    }
-    // ... and run on streams of the highest priority; the row sort's stream has the default one
-    const int rc = scatter_prepare_aside(ws, FS, row_dev, total, hotn, st);
-    if (rc != CAFE_OK && insert_mode != CAFE_INSERT_SEQUENTIAL) cafe_internal_presort(h, nullptr, 0, nullptr, nullptr, st);   // withdrawn
-    return rc;
-}
-static int scatter_join(CafeEmbedWorkspace* ws, cudaStream_t st) {
-    return cudaStreamWaitEvent(st, ws->ev_join, 0) == cudaSuccess ? CAFE_OK : fail_cuda("scatter join wait");
+    if (insert_mode == CAFE_INSERT_SEQUENTIAL) { ws->keys_of = nullptr; return scatter_prepare(ws, FS, row_dev, total, st); }
+    // row keys left by cafe_embed_resolve for exactly these lookups
+    const bool have = ws->keys_of == gid_dev && ws->keys_total == total;
+    if (!have) { row_keys(ws, FS, row_dev, total, st); ws->keys_of = nullptr; }
+    const CafeSortDesc rows = row_sort_desc(ws, FS, total);
+    cafe_internal_presort(h, gid_dev, total, &rows, st);
+    return CAFE_OK;
 }
 
 // The whole post-backward part of one training step for `nfields` fields, in the reference's order:
@@ -1044,8 +1037,8 @@ static int embed_backward_impl(void* h, const float* grad_dev, int64_t field_str
         if (cudaStreamWaitEvent(st, gate_event, 0) != cudaSuccess) return fail_cuda("gate wait");
         gated = false;
     }
-    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, hotn, insert_mode, st);
-    if (rc != CAFE_OK) { scatter_join(ws, st); return rc; }
+    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, insert_mode, st);
+    if (rc != CAFE_OK) return rc;
     const int early = gated ? gate_field : nfields;
     rc = importance_range(ws, grad_dev, field_stride, sample_stride, 0, early, B, D, ws->imp, st);
     if (rc == CAFE_OK && gated) {
@@ -1058,8 +1051,7 @@ static int embed_backward_impl(void* h, const float* grad_dev, int64_t field_str
         if (rc == CAFE_OK) cafe_internal_set_gate(h, gate_field, ws->ev_late);
     }
     if (rc != CAFE_OK) {
-        cafe_internal_presort(h, nullptr, 0, nullptr, nullptr, st);   // withdraws the sorts started above
-        scatter_join(ws, st);
+        cafe_internal_presort(h, nullptr, 0, nullptr, st);   // withdraws the sorts started above
         return rc;
     }
     int seg[CAFE_MAX_SEGMENTS + 1];
@@ -1068,7 +1060,7 @@ static int embed_backward_impl(void* h, const float* grad_dev, int64_t field_str
     int status = cafe_internal_insert(h, gid_dev, ws->imp, seg, nfields, mask, ws->post_row, insert_mode, st);
     cafe_internal_set_gate(h, -1, nullptr);
     if (gated) cudaStreamWaitEvent(st, ws->ev_late, 0);   // whatever the insert did: the scatter reads every field
-    rc = scatter_join(ws, st);
+    rc = cafe_internal_sort_join(h, st);
     if (status != CAFE_OK && status != CAFE_ERR_NOCONVERGE && status != CAFE_ERR_RESET_UNDERFLOW) return status;
     if (rc != CAFE_OK) return rc;
     rc = cafe_migrate(h, ids_dev, ids_are_int64, mask, ws->post_row, nfields, B, f_offset, hash_size, weight_hash, weight_high,
@@ -1176,7 +1168,7 @@ int cafe_embed_backward_begin(void* h, const uint32_t* gid_dev, const int32_t* r
     if (total > ws->cap) return CAFE_ERR_CAPACITY;
     if (total == 0) return CAFE_OK;
     ws->begun_gid = nullptr;
-    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, hotn, insert_mode, (cudaStream_t)stream);
+    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, insert_mode, (cudaStream_t)stream);
     if (rc != CAFE_OK) return rc;
     ws->begun_gid = gid_dev; ws->begun_row = row_dev; ws->begun_total = (int)total; ws->begun_mode = insert_mode;
     return CAFE_OK;
@@ -1200,10 +1192,10 @@ int cafe_embed_backward_imp(void* h, const float* grad_dev, int64_t field_stride
     int rc = scatter_check(h, &FS, grad_dev, field_stride, sample_stride, row_dev, nfields, B, hash_size, weight_hash,
                            weight_high, hotn, D);
     if (rc != CAFE_OK) return rc;
-    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, hotn, insert_mode, (cudaStream_t)stream);
-    if (rc != CAFE_OK) { scatter_join(ws, (cudaStream_t)stream); return rc; }
+    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, insert_mode, (cudaStream_t)stream);
+    if (rc != CAFE_OK) return rc;
     int status = cafe_internal_insert(h, gid_dev, imp_dev, seg, nfields, mask, ws->post_row, insert_mode, (cudaStream_t)stream);
-    rc = scatter_join(ws, (cudaStream_t)stream);
+    rc = cafe_internal_sort_join(h, (cudaStream_t)stream);
     if (status != CAFE_OK && status != CAFE_ERR_NOCONVERGE && status != CAFE_ERR_RESET_UNDERFLOW) return status;
     if (rc != CAFE_OK) return rc;
     rc = cafe_migrate(h, ids_dev, ids_are_int64, mask, ws->post_row, nfields, B, f_offset, hash_size, weight_hash, weight_high,
@@ -1288,15 +1280,15 @@ int cafe_embed_backward_norms(void* h, const float* grad_dev, int64_t field_stri
     int rc = scatter_check(h, &FS, grad_dev, field_stride, sample_stride, row_dev, nfields, B, hash_size, weight_hash,
                            weight_high, hotn, D);
     if (rc != CAFE_OK) return rc;
-    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, hotn, insert_mode, st);
-    if (rc != CAFE_OK) { scatter_join(ws, st); return rc; }
+    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, insert_mode, st);
+    if (rc != CAFE_OK) return rc;
     { CAFE_PROF(CAFE_P_FIELDSUM, st); k_field_sum<<<nfields, 1024, 0, st>>>(norm_dev, B, ws->totals); }
     { CAFE_PROF(CAFE_P_IMPORTANCE, st); k_importance<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(norm_dev, ws->totals, B,
                                                                                                     (int)total, ws->imp); }
     int seg[CAFE_MAX_SEGMENTS + 1];
     for (int f = 0; f <= nfields; ++f) seg[f] = f * B;
     int status = cafe_internal_insert(h, gid_dev, ws->imp, seg, nfields, ws->mask, ws->post_row, insert_mode, st);
-    rc = scatter_join(ws, st);
+    rc = cafe_internal_sort_join(h, st);
     if (status != CAFE_OK && status != CAFE_ERR_NOCONVERGE && status != CAFE_ERR_RESET_UNDERFLOW) return status;
     if (rc != CAFE_OK) return rc;
     rc = cafe_migrate(h, ids_dev, ids_are_int64, ws->mask, ws->post_row, nfields, B, f_offset, hash_size, weight_hash, weight_high,

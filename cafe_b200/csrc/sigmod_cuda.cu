@@ -54,8 +54,8 @@ struct SgHandle {
     SgBucket* b = nullptr;
     uint32_t* ring = nullptr;
     SgState* st = nullptr;
-    uint32_t *key = nullptr, *key_tmp = nullptr, *skey = nullptr, *sgid = nullptr;
-    int32_t *pos_tmp = nullptr, *ord = nullptr, *start = nullptr, *rank = nullptr, *blk = nullptr, *sort_scratch = nullptr;
+    uint2 *ent = nullptr, *ent_tmp = nullptr;   // lookups by (bucket, position): (id, position), and pairs between two sort passes
+    int32_t *start = nullptr, *rank = nullptr, *blk = nullptr, *sort_scratch = nullptr;
     float* simp = nullptr;
     uint8_t* cand = nullptr;
     double* partial = nullptr;
@@ -224,20 +224,9 @@ __global__ void k_sg_mass_end(SgState* st, const double* __restrict__ partial, i
 }
 
 // ---- the two replays ---------------------------------------------------------------------------------------
-__global__ void k_sg_keys(const uint32_t* __restrict__ gid, int n, int s, uint32_t* __restrict__ key) {
+__global__ void k_sg_gather_counts(const float* __restrict__ imp, const uint2* __restrict__ ent, int n, float* __restrict__ simp) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) key[i] = gid[i] % (uint32_t)s;   // :22-24
-}
-__global__ void k_sg_starts(const uint32_t* __restrict__ skey, int M, int nb, int32_t* __restrict__ start) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > M) return;
-    const int lo = (i == 0) ? 0 : (int)skey[i - 1] + 1;
-    const int hi = (i == M) ? nb : (int)skey[i];
-    for (int k = lo; k <= hi; ++k) start[k] = i;
-}
-__global__ void k_sg_gather_counts(const float* __restrict__ imp, const int32_t* __restrict__ ord, int n, float* __restrict__ simp) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) simp[i] = imp[ord[i]];
+    if (i < n) simp[i] = imp[ent[i].y];
 }
 
 // Insert (sketch.cpp:89-123) of one lookup into a bucket held in registers.  COMMIT = false: pass A (a candidate
@@ -288,7 +277,7 @@ __device__ __forceinline__ void sg_insert(SgBucket& b, uint32_t x, float v, floa
 
 template <bool COMMIT>
 __global__ void __launch_bounds__(SG_TPB) k_sg_pass(SgBucket* __restrict__ tb, int s, int k, const int32_t* __restrict__ start,
-                                                    const int32_t* __restrict__ ord, const uint32_t* __restrict__ sgid,
+                                                    const uint2* __restrict__ ent,
                                                     const float* __restrict__ simp, uint8_t* __restrict__ cand,
                                                     const int32_t* __restrict__ rank, const SgState* __restrict__ st,
                                                     const uint32_t* __restrict__ ring, uint32_t mask, int32_t* __restrict__ out) {
@@ -301,7 +290,7 @@ __global__ void __launch_bounds__(SG_TPB) k_sg_pass(SgBucket* __restrict__ tb, i
     const int32_t q_size = COMMIT ? st->q_size : 0;
     const uint32_t q_head = COMMIT ? st->q_head : 0u;
     for (int i = i0; i < i1; ++i)
-        sg_insert<COMMIT>(b, sgid[i], simp ? simp[i] : 1.0f, kf, ord[i], cand, rank, q_size, q_head, ring, mask, out);
+        sg_insert<COMMIT>(b, ent[i].x, simp ? simp[i] : 1.0f, kf, (int)ent[i].y, cand, rank, q_size, q_head, ring, mask, out);
     if (COMMIT) tb[key] = b;
 }
 
@@ -390,7 +379,7 @@ static int sg_fail(const char* where) {
     return CAFE_ERR_CUDA;
 }
 static void sg_release(SgHandle* H) {
-    void* ptrs[] = {H->b, H->ring, H->st, H->key, H->key_tmp, H->skey, H->sgid, H->pos_tmp, H->ord, H->start, H->rank, H->blk,
+    void* ptrs[] = {H->b, H->ring, H->st, H->ent, H->ent_tmp, H->start, H->rank, H->blk,
                     H->sort_scratch, H->simp, H->cand, H->partial};
     for (void* p : ptrs) if (p) cudaFree(p);
     delete H;
@@ -412,9 +401,8 @@ int cafe_sigmod_create(void** out, int lim, int threshold, double decay_rate, in
     const size_t nblk = (size_t)((lim > max_lookups ? lim : max_lookups) / SG_BLK + 2);
     auto A = [&](void** p, size_t n) { if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1); };
     A((void**)&H->b, sizeof(SgBucket) * (size_t)lim); A((void**)&H->ring, 4 * (size_t)rc); A((void**)&H->st, sizeof(SgState));
-    A((void**)&H->key, 4 * M); A((void**)&H->key_tmp, 4 * M); A((void**)&H->skey, 4 * M); A((void**)&H->sgid, 4 * M);
-    A((void**)&H->pos_tmp, 4 * M); A((void**)&H->ord, 4 * M); A((void**)&H->start, 4 * ((size_t)lim + 1)); A((void**)&H->rank, 4 * M);
-    A((void**)&H->blk, 4 * nblk); A((void**)&H->sort_scratch, 4 * cafe_rs_scratch_elems(max_lookups)); A((void**)&H->simp, 4 * M);
+    A((void**)&H->ent, sizeof(uint2) * M); A((void**)&H->ent_tmp, sizeof(uint2) * M); A((void**)&H->start, 4 * ((size_t)lim + 1)); A((void**)&H->rank, 4 * M);
+    A((void**)&H->blk, 4 * nblk); A((void**)&H->sort_scratch, 4 * cafe_rs_scratch_elems()); A((void**)&H->simp, 4 * M);
     A((void**)&H->cand, M > (size_t)lim + 1 ? M : (size_t)lim + 1); A((void**)&H->partial, 8 * nblk);
     if (e == cudaSuccess) e = cudaMemset(H->b, 0, sizeof(SgBucket) * (size_t)lim);
     if (e == cudaSuccess) {
@@ -481,22 +469,22 @@ int cafe_sigmod_insert(void* h, const uint32_t* gid_dev, const float* imp_dev, i
     if (imp_dev) k_sg_mass<<<npb, SG_TPB, 0, st>>>(imp_dev, n, H->partial);
     k_sg_mass_end<<<1, 1, 0, st>>>(H->st, H->partial, npb, n, imp_dev ? 0 : 1);
     // lookups by (bucket, position)
-    k_sg_keys<<<sg_blocks(n), SG_TPB, 0, st>>>(gid_dev, n, s, H->key);
-    int bits = 1;
-    while ((1ll << bits) < s) ++bits;
-    CafeKeySource src;
-    src.key = H->key; src.gid = nullptr; src.nb = 0;
-    cudaError_t e = cafe_radix_sort(src, nullptr, H->key_tmp, H->pos_tmp, H->skey, H->ord, n, bits, H->sort_scratch, gid_dev, H->sgid, st);
+    CafeSortBatch batch;
+    batch.count = 1;
+    CafeSortDesc& D = batch.d[0];
+    memset(&D, 0, sizeof(D));
+    D.in = gid_dev; D.hashed = 2; D.mod.n = s; D.n = n; D.tmp = H->ent_tmp; D.out = H->ent; D.start = H->start;
+    D.scratch = H->sort_scratch;
+    cudaError_t e = cafe_radix_sort(batch, st);
     if (e != cudaSuccess) { cafe_internal_set_error(cudaGetErrorString(e)); return CAFE_ERR_CUDA; }
-    k_sg_starts<<<sg_blocks((int64_t)n + 1), SG_TPB, 0, st>>>(H->skey, n, s, H->start);
-    if (imp_dev) k_sg_gather_counts<<<sg_blocks(n), SG_TPB, 0, st>>>(imp_dev, H->ord, n, H->simp);
+    if (imp_dev) k_sg_gather_counts<<<sg_blocks(n), SG_TPB, 0, st>>>(imp_dev, H->ent, n, H->simp);
     const float* simp = imp_dev ? H->simp : nullptr;
     cudaMemsetAsync(H->cand, 0, (size_t)n, st);
-    k_sg_pass<false><<<sg_blocks(s), SG_TPB, 0, st>>>(H->b, s, H->k, H->start, H->ord, H->sgid, simp, H->cand, nullptr, H->st, H->ring,
+    k_sg_pass<false><<<sg_blocks(s), SG_TPB, 0, st>>>(H->b, s, H->k, H->start, H->ent, simp, H->cand, nullptr, H->st, H->ring,
                                                       H->ring_mask, nullptr);
     k_sg_rank_count<<<npb, SG_TPB, 0, st>>>(H->cand, n, H->blk);
     k_sg_rank_write<<<npb, SG_TPB, 0, st>>>(H->cand, n, H->blk, H->rank, H->st);
-    k_sg_pass<true><<<sg_blocks(s), SG_TPB, 0, st>>>(H->b, s, H->k, H->start, H->ord, H->sgid, simp, H->cand, H->rank, H->st, H->ring,
+    k_sg_pass<true><<<sg_blocks(s), SG_TPB, 0, st>>>(H->b, s, H->k, H->start, H->ent, simp, H->cand, H->rank, H->st, H->ring,
                                                      H->ring_mask, mask_out_dev);
     k_sg_end<<<1, 1, 0, st>>>(H->st);
     return sg_fail("cafe_sigmod_insert");

@@ -45,6 +45,28 @@ CAFE_HD int32_t cafe_hash(uint32_t x, int32_t n) {
     return (int32_t)(((int64_t)x * 1000000007LL) % (int64_t)n);
 }
 
+// The same remainder by a divisor that is known ahead: q = high word of v * floor(2^64 / n) is the quotient or one less
+// (v < 2^62), so one conditional subtraction ends it.  A dozen instructions instead of the hundred of a 64-bit
+// division; every kernel that hashes ids takes it.
+struct CafeMod { uint64_t magic; int32_t n; };
+static inline CafeMod cafe_mod_of(int32_t n) {
+    CafeMod m;
+    m.n = n;
+    m.magic = n > 1 ? (uint64_t)((((unsigned __int128)1) << 64) / (unsigned)n) : 0;
+    return m;
+}
+CAFE_HD int32_t cafe_hash(uint32_t x, const CafeMod& m) {
+    const uint64_t v = (uint64_t)x * 1000000007ull;
+#if defined(__CUDA_ARCH__)
+    const uint32_t q = (uint32_t)__umul64hi(v, m.magic);
+#else
+    const uint32_t q = (uint32_t)(uint64_t)(((unsigned __int128)v * m.magic) >> 64);
+#endif
+    uint32_t r = (uint32_t)v - q * (uint32_t)m.n;   // below 2n, whatever wrapped
+    if (r >= (uint32_t)m.n) r -= (uint32_t)m.n;
+    return m.n > 1 ? (int32_t)r : 0;
+}
+
 CAFE_HD uint32_t cafe_float_bits(float f) {
 #if defined(__CUDA_ARCH__)
     return __float_as_uint(f);
@@ -208,6 +230,14 @@ struct alignas(16) CafeFn { int32_t a, b, np, pad; };   // FIFO size transfer s 
 #define CAFE_TL_BLOCK 1024    // positions (resp. ops) handled by one block of the timeline kernels
 #define CAFE_TL_GROUP 64      // positions per entry of the coarse index into the op list
 
+#if defined(__CUDACC__)
+#define CAFE_ORD_STRIDE 2
+#else
+#define CAFE_ORD_STRIDE 1
+#endif
+CAFE_HD int32_t cafe_ord(const int32_t* ord, int64_t i) { return ord[i * CAFE_ORD_STRIDE]; }
+CAFE_HD uint32_t cafe_sid(const uint32_t* sgid, int64_t i) { return sgid[i * CAFE_ORD_STRIDE]; }
+
 // per-lookup result flags (one byte written by the main pass, one by the LRU pass)
 enum { CAFE_F_MISS = 1, CAFE_F_POP0 = 2, CAFE_F_POP1 = 4, CAFE_F_CROSS = 8, CAFE_F_GOT = 16 };
 // per-bucket replay state kept between rounds
@@ -226,6 +256,8 @@ struct CafeJob {
     int32_t nseg;
     int32_t seg_off[CAFE_MAX_SEGMENTS + 1];
     // positions ordered by (main bucket, position) and by (LRU bucket, position); bucket ranges
+    // (ids and positions of an order are CAFE_ORD_STRIDE words apart: the CUDA build keeps them as pairs, so that a replay
+    // loads both at once and the sort stores both at once)
     const int32_t* ord1;
     const int32_t* start1;   // [n1+1] bucket ranges in ord1 (whole call)
     const int32_t* beg1;     // [n1]   first entry of each bucket that is >= begin
@@ -244,6 +276,7 @@ struct CafeJob {
     const CafeLruBucket* lru_in;
     CafeLruBucket* lru_out;
     int32_t n1, n2;
+    CafeMod mod1, mod2;      // hashes into the two tables
     float thr;
     uint32_t gflip;
     int32_t t0;
@@ -357,15 +390,15 @@ CAFE_HD uint32_t cafe_old_mflag(const CafeJob& J, int p) { return J.first_round 
 CAFE_HD void cafe_route_position(const CafeJob& J, int p) {
     if (!(J.mflag[p] & CAFE_F_MISS)) return;   // a lookup that hit the main table has no event
     const CafeEvent e = J.ev[p];
-    if (e.kind == CAFE_EV_VICTIM) J.nxt[p] = CAFE_ATOMIC_EXCH(&J.head[cafe_hash(e.x, J.n1)], p);
-    else if (e.kind == CAFE_EV_OWN) J.mark_own[cafe_hash(e.x, J.n1)] = 1;
+    if (e.kind == CAFE_EV_VICTIM) J.nxt[p] = CAFE_ATOMIC_EXCH(&J.head[cafe_hash(e.x, J.mod1)], p);
+    else if (e.kind == CAFE_EV_OWN) J.mark_own[cafe_hash(e.x, J.mod1)] = 1;
 }
 
 // the event of position p no longer exists (its lookup hits the main table now, or its LRU replay produces none):
 // the main bucket it would have landed in replays without it
 CAFE_HD void cafe_withdraw_event(const CafeJob& J, int p) {
     const CafeEvent o = J.ev[p];
-    if (o.kind != CAFE_EV_NONE) J.mark_out1[cafe_hash(o.x, J.n1)] = 1;
+    if (o.kind != CAFE_EV_NONE) J.mark_out1[cafe_hash(o.x, J.mod1)] = 1;
     J.ev[p].kind = CAFE_EV_NONE;
     J.res->changed = 1;
 }
@@ -376,11 +409,11 @@ CAFE_HD void cafe_withdraw_event(const CafeJob& J, int p) {
 // `mark_next1` is the array the next round's main pass reads.
 CAFE_HD void cafe_mark_cut_position(const CafeJob& J, int p, uint8_t* mark_next1) {
     const uint32_t x = J.gid[p];
-    mark_next1[cafe_hash(x, J.n1)] = 1;
+    mark_next1[cafe_hash(x, J.mod1)] = 1;
     if (J.mflag[p] & CAFE_F_MISS) {
-        J.mark_c2[cafe_hash(x, J.n2)] = 1;
+        J.mark_c2[cafe_hash(x, J.mod2)] = 1;
         const CafeEvent e = J.ev[p];
-        if (e.kind != CAFE_EV_NONE) mark_next1[cafe_hash(e.x, J.n1)] = 1;
+        if (e.kind != CAFE_EV_NONE) mark_next1[cafe_hash(e.x, J.mod1)] = 1;
     }
 }
 
@@ -439,7 +472,7 @@ struct CafeMainReplay {
 #pragma unroll
                 for (int j = 0; j < CAFE_CAND; ++j) if (j < ncand) J.post_row[cand_p[j]] = cafe_probe_hot(b, cand_x[j]);
             } else {
-                for (int j = i_first; j < i_cur; ++j) { int q = J.ord1[j]; J.post_row[q] = cafe_probe_hot(b, J.gid[q]); }
+                for (int j = i_first; j < i_cur; ++j) { int q = cafe_ord(J.ord1, j); J.post_row[q] = cafe_probe_hot(b, J.gid[q]); }
             }
         }
         dirty = false; ncand = 0; i_first = i_cur;
@@ -502,7 +535,7 @@ struct CafeMainReplay {
                 if (nf != old_flag) J.mflag[p] = (uint8_t)nf;
                 if (!J.first_round) {
                     if (old_kind != CAFE_EV_NONE) cafe_withdraw_event(J, p);
-                    if (old_flag & CAFE_F_MISS) { J.mark2[cafe_hash(x, J.n2)] = 1; J.res->miss_changed = 1; }   // its LRU bucket loses this visitor
+                    if (old_flag & CAFE_F_MISS) { J.mark2[cafe_hash(x, J.mod2)] = 1; J.res->miss_changed = 1; }   // its LRU bucket loses this visitor
                 }
             }
         } else {
@@ -510,11 +543,11 @@ struct CafeMainReplay {
             if (J.final_pass) { if (J.lflag[p] & CAFE_F_GOT) note_cand(p, x); }
             else {
                 if (old_flag != CAFE_F_MISS) J.mflag[p] = CAFE_F_MISS;   // goes to the LRU stage; that pass writes lflag
-                if (!J.first_round && !(old_flag & CAFE_F_MISS)) { J.mark2[cafe_hash(x, J.n2)] = 1; J.res->miss_changed = 1; }   // new visitor
+                if (!J.first_round && !(old_flag & CAFE_F_MISS)) { J.mark2[cafe_hash(x, J.mod2)] = 1; J.res->miss_changed = 1; }   // new visitor
             }
             if (old_kind == CAFE_EV_OWN) {   // believed: this lookup promotes its own id into this bucket
                 apply_event(J, p);
-                if (!J.final_pass) J.mark2[cafe_hash(x, J.n2)] = 1;   // the LRU bucket reads ins_res[p]
+                if (!J.final_pass) J.mark2[cafe_hash(x, J.mod2)] = 1;   // the LRU bucket reads ins_res[p]
             }
         }
         ++i_cur;
@@ -534,7 +567,7 @@ CAFE_HD void cafe_main_pass_bucket(const CafeJob& J, int k) {
     int i = J.beg1[k];
     if (!R.init(J, k, i)) return;
     for (; i < iend; ++i) {
-        const int p = J.ord1[i];
+        const int p = cafe_ord(J.ord1, i);
         if (p >= J.limit) break;
         R.feed(J, p, J.gid[p], cafe_count_of(J, p), cafe_old_kind(J, p), cafe_old_mflag(J, p));
     }
@@ -582,10 +615,10 @@ struct CafeLruReplay {
             else same = (o.kind == kind && o.x == x && o.dic == dic && cafe_float_bits(o.cnt) == cafe_float_bits(cnt));
             if (same) return;
             J.res->changed = 1;
-            if (o.kind != CAFE_EV_NONE) J.mark_out1[cafe_hash(o.x, J.n1)] = 1;   // the old event's target loses it
+            if (o.kind != CAFE_EV_NONE) J.mark_out1[cafe_hash(o.x, J.mod1)] = 1;   // the old event's target loses it
             if (kind == CAFE_EV_NONE) { J.ev[p].kind = CAFE_EV_NONE; return; }
         }
-        J.mark_out1[cafe_hash(x, J.n1)] = 1;   // the new event's target
+        J.mark_out1[cafe_hash(x, J.mod1)] = 1;   // the new event's target
         CafeEvent e;
         e.x = x; e.cnt = cnt; e.dic = dic; e.kind = kind;
         J.ev[p] = e;
@@ -665,7 +698,7 @@ CAFE_HD void cafe_lru_pass_bucket(const CafeJob& J, int k) {
     if (!R.init(J, k)) return;
     const int jend = J.start2[k + 1];
     for (int j = J.beg2[k]; j < jend; ++j) {
-        const int p = J.ord2[j];
+        const int p = cafe_ord(J.ord2, j);
         if (p >= J.limit) break;
         if (!(J.mflag[p] & CAFE_F_MISS)) continue;
         R.feed(J, p, J.gid[p], cafe_count_of(J, p));
@@ -677,7 +710,7 @@ CAFE_HD void cafe_lru_pass_bucket(const CafeJob& J, int k) {
 CAFE_HD int32_t cafe_advance_cursor(const int32_t* ord, int32_t lo, int32_t hi, int32_t limit) {
     while (lo < hi) {
         const int32_t mid = (lo + hi) >> 1;
-        if (ord[mid] < limit) lo = mid + 1; else hi = mid;
+        if (cafe_ord(ord, mid) < limit) lo = mid + 1; else hi = mid;
     }
     return lo;
 }
@@ -779,8 +812,8 @@ CAFE_HD void cafe_tl_finish_op(const CafeJob& J, int32_t j, int32_t n, const Caf
         const int p = J.tl_slot[j] >> 1;
         const uint32_t f = cafe_eff_flag(J, p);
         if (s > 0 || (f & CAFE_F_GOT)) {
-            if (f & CAFE_F_MISS) J.mark_c2[cafe_hash(J.gid[p], J.n2)] = 1;
-            else J.mark_out1[cafe_hash(J.gid[p], J.n1)] = 1;
+            if (f & CAFE_F_MISS) J.mark_c2[cafe_hash(J.gid[p], J.mod2)] = 1;
+            else J.mark_out1[cafe_hash(J.gid[p], J.mod1)] = 1;
         }
     }
     // the first round believed an untouched FIFO everywhere: a push or a successful pop contradicts that

@@ -53,7 +53,7 @@ __global__ void k_fills(const CafeFills F) {
     }
 }
 
-__global__ void k_query(const CafeMainBucket* __restrict__ mb, int n1, const uint32_t* __restrict__ gid, int n,
+__global__ void k_query(const CafeMainBucket* __restrict__ mb, const CafeMod n1, const uint32_t* __restrict__ gid, int n,
                         int32_t* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -70,7 +70,7 @@ __global__ void k_query(const CafeMainBucket* __restrict__ mb, int n1, const uin
     out[i] = r ? -r : (int32_t)x;
 }
 
-__global__ void k_post_query(const CafeMainBucket* __restrict__ mb, int n1, const uint32_t* __restrict__ gid, int n,
+__global__ void k_post_query(const CafeMainBucket* __restrict__ mb, const CafeMod n1, const uint32_t* __restrict__ gid, int n,
                              const int32_t* __restrict__ mask, int32_t* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -79,25 +79,13 @@ __global__ void k_post_query(const CafeMainBucket* __restrict__ mb, int n1, cons
     out[i] = r;
 }
 
-// start[k] = first sorted index whose key is >= k, for k in [0, nb]
-// (also zeroes the two counters of the long-bucket list that k_find_hot, the next launch, fills)
-__global__ void k_bucket_starts(const uint32_t* __restrict__ skey, int M, int nb, int32_t* __restrict__ start,
-                                int32_t* __restrict__ hot_count) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 2) hot_count[i] = 0;
-    if (i > M) return;
-    const int lo = (i == 0) ? 0 : (int)skey[i - 1] + 1;
-    const int hi = (i == M) ? nb : (int)skey[i];
-    for (int k = lo; k <= hi; ++k) start[k] = i;
-}
-
 // counts in bucket order, so that the replay kernels stream them beside the sorted positions and ids
 __global__ void k_gather_counts(const float* __restrict__ imp, const int32_t* __restrict__ ord1, const int32_t* __restrict__ ord2,
                                 int M, float* __restrict__ simp1, float* __restrict__ simp2) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
-    simp1[i] = imp[ord1[i]];
-    simp2[i] = imp[ord2[i]];
+    simp1[i] = imp[cafe_ord(ord1, i)];
+    simp2[i] = imp[cafe_ord(ord2, i)];
 }
 
 // Buckets with at most CAFE_LONG lookups are replayed by their own thread.  Longer ones (the ids at
@@ -125,27 +113,34 @@ struct CafeHot {
     const uint8_t* flag;
     int32_t cap2;   // capacity of the second region
 };
-// (also sets every bucket's flag, listed or not, and its cursor beg[k] = start[k])
-__global__ void k_find_hot(const int32_t* __restrict__ start, int nb, int hot_len, int long_len, int cap2, int32_t* list,
-                           int32_t* count, uint8_t* flag, int32_t* __restrict__ beg) {
+// (also sets every bucket's flag, listed or not, and its cursor beg[k] = start[k]; blockIdx.y = table)
+struct CafeFindHot {
+    const int32_t* start;
+    int32_t nb, hot_len, long_len;
+    int32_t *list, *count;
+    uint8_t* flag;
+    int32_t* beg;
+};
+__global__ void k_find_hot(const CafeFindHot A, const CafeFindHot B) {
+    const CafeFindHot& T = blockIdx.y == 0 ? A : B;
     int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nb) return;
-    const int s0 = start[k];
-    const int len = start[k + 1] - s0;
-    beg[k] = s0;
+    if (k >= T.nb) return;
+    const int s0 = T.start[k];
+    const int len = T.start[k + 1] - s0;
+    T.beg[k] = s0;
     uint8_t listed = 0;
-    if (len > long_len) {
+    if (len > T.long_len) {
         bool placed = false;
-        if (len > hot_len) {
-            const int idx = atomicAdd(&count[0], 1);
-            if (idx < CAFE_HOT_CAP) { list[idx] = k; listed = 1; placed = true; }
+        if (len > T.hot_len) {
+            const int idx = atomicAdd(&T.count[0], 1);
+            if (idx < CAFE_HOT_CAP) { T.list[idx] = k; listed = 1; placed = true; }
         }
         if (!placed) {
-            const int idx = atomicAdd(&count[1], 1);
-            if (idx < cap2) { list[CAFE_HOT_CAP + idx] = k; listed = 1; }
+            const int idx = atomicAdd(&T.count[1], 1);
+            if (idx < T.nb) { T.list[CAFE_HOT_CAP + idx] = k; listed = 1; }
         }
     }
-    flag[k] = listed;
+    T.flag[k] = listed;
 }
 // next listed bucket for this warp (lane 0 owns it; -1 = none left); the cursor is zeroed with the round result
 __device__ __forceinline__ int cafe_next_listed(const CafeHot& H, int32_t* cursor, int nb) {
@@ -233,7 +228,7 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                 float c = 1.0f;
                 if (e < t0 + tn) {
                     const int idx = iL + (e - pL);   // position, id and count come from the same sorted index
-                    p = J.ord1[idx]; x = J.sgid1[idx];
+                    p = cafe_ord(J.ord1, idx); x = cafe_sid(J.sgid1, idx);
                     if (J.simp1) c = J.simp1[idx];
                     if (!J.first_round && p < J.limit) kf = cafe_old_kind(J, p) | (cafe_old_mflag(J, p) << 8);
                 }
@@ -261,11 +256,11 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
         int hslot = 0, hbound = 0;
         // two-deep software pipeline: positions of chunk n+2 and the per-lookup data of chunk n+1 are
         // requested before chunk n is processed, so a long bucket pays one load latency, not one per chunk
-        int p_nx = (s + lane < e) ? J.ord1[s + lane] : INT32_MAX;
-        int p_n2 = (s + 32 + lane < e) ? J.ord1[s + 32 + lane] : INT32_MAX;
+        int p_nx = (s + lane < e) ? cafe_ord(J.ord1, s + lane) : INT32_MAX;
+        int p_n2 = (s + 32 + lane < e) ? cafe_ord(J.ord1, s + 32 + lane) : INT32_MAX;
         uint32_t x_nx = 0, ok_nx = CAFE_EV_NONE, of_nx = 0;
         float c_nx = 1.0f;
-        if (s + lane < e) { x_nx = J.sgid1[s + lane]; if (J.simp1) c_nx = J.simp1[s + lane]; }
+        if (s + lane < e) { x_nx = cafe_sid(J.sgid1, s + lane); if (J.simp1) c_nx = J.simp1[s + lane]; }
         // (the final pass asks of every miss whether the LRU stage handed it a row: that flag byte rides in bits 8-15)
         if (p_nx < J.limit) { ok_nx = cafe_old_kind(J, p_nx); of_nx = cafe_old_mflag(J, p_nx); if (J.final_pass) of_nx |= (uint32_t)J.lflag[p_nx] << 8; }
         // Number of chunks in a row that went through the calm whole-chunk path.  A calm chunk that ends on a multiple
@@ -315,11 +310,11 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const int i0 = gb + 32 * q + lane, i1 = i0 + 128;
-                    Ap[q] = i0 < e ? J.ord1[i0] : INT32_MAX;
-                    Bp[q] = i1 < e ? J.ord1[i1] : INT32_MAX;
+                    Ap[q] = i0 < e ? cafe_ord(J.ord1, i0) : INT32_MAX;
+                    Bp[q] = i1 < e ? cafe_ord(J.ord1, i1) : INT32_MAX;
                     Ax[q] = 0; Ac[q] = 1.0f; Bx[q] = 0; Bc[q] = 1.0f;
-                    if (i0 < e) { Ax[q] = J.sgid1[i0]; if (J.simp1) Ac[q] = J.simp1[i0]; }
-                    if (i1 < e) { Bx[q] = J.sgid1[i1]; if (J.simp1) Bc[q] = J.simp1[i1]; }
+                    if (i0 < e) { Ax[q] = cafe_sid(J.sgid1, i0); if (J.simp1) Ac[q] = J.simp1[i0]; }
+                    if (i1 < e) { Bx[q] = cafe_sid(J.sgid1, i1); if (J.simp1) Bc[q] = J.simp1[i1]; }
                     Cp[q] = INT32_MAX; Cx[q] = 0; Cc[q] = 1.0f; Cok[q] = CAFE_EV_NONE; Cof[q] = 0; Bok[q] = CAFE_EV_NONE; Bof[q] = 0;
                 }
 #pragma unroll
@@ -352,7 +347,7 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                     _Pragma("unroll") for (int q = 0; q < 4; ++q) {                                                       \
                         const int i2 = gb + 256 + 32 * q + lane;                                                          \
                         Y##p[q] = INT32_MAX; Y##x[q] = 0; Y##c[q] = 1.0f;                                                 \
-                        if (i2 < e) { Y##p[q] = J.ord1[i2]; Y##x[q] = J.sgid1[i2]; if (J.simp1) Y##c[q] = J.simp1[i2]; }  \
+                        if (i2 < e) { Y##p[q] = cafe_ord(J.ord1, i2); Y##x[q] = cafe_sid(J.sgid1, i2); if (J.simp1) Y##c[q] = J.simp1[i2]; }  \
                         X##ok[q] = CAFE_EV_NONE; X##of[q] = 0;                                                            \
                         if (X##p[q] < J.limit) { X##ok[q] = cafe_old_kind(J, X##p[q]); X##of[q] = cafe_old_mflag(J, X##p[q]); } \
                     }                                                                                                     \
@@ -369,7 +364,7 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                             if (C##of[q] != 0) J.mflag[C##p[q]] = 0;                                                      \
                             if (!J.first_round) {                                                                         \
                                 if (C##ok[q] != CAFE_EV_NONE) cafe_withdraw_event(J, C##p[q]);                            \
-                                if (C##of[q] & CAFE_F_MISS) { J.mark2[cafe_hash(C##x[q], J.n2)] = 1; J.res->miss_changed = 1; } \
+                                if (C##of[q] & CAFE_F_MISS) { J.mark2[cafe_hash(C##x[q], J.mod2)] = 1; J.res->miss_changed = 1; } \
                             }                                                                                             \
                         }                                                                                                 \
                     }                                                                                                     \
@@ -392,8 +387,8 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                 {                                                                                                         \
                     _Pragma("unroll") for (int q = 0; q < 4; ++q) {                                                       \
                         const int i2 = gb + 256 + 32 * q + lane, i2c = min(i2, e - 1);                                    \
-                        const int yp = J.ord1[i2c];                                                                       \
-                        Y##x[q] = J.sgid1[i2c];                                                                           \
+                        const int yp = cafe_ord(J.ord1, i2c);                                                                       \
+                        Y##x[q] = cafe_sid(J.sgid1, i2c);                                                                           \
                         Y##c[q] = imp1[i2c];                                                                              \
                         Y##p[q] = i2 < e ? yp : INT32_MAX;                                                                \
                     }                                                                                                     \
@@ -441,7 +436,7 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                 if (gb != base) {
                     if (J.memo1 && g_start == base && gb - base >= 512 && lane == 0) {   // (walked, not jumped: remember it)
                         CafeCalmMemo mm;
-                        mm.serial = J.serial; mm.i0 = base; mm.i1 = gb; mm.p_last = J.ord1[gb - 1];
+                        mm.serial = J.serial; mm.i0 = base; mm.i1 = gb; mm.p_last = cafe_ord(J.ord1, gb - 1);
                         mm.acc_in = acc_in; mm.acc_out = __float_as_uint(acc); mm.x = hx; mm.slot = hslot;
                         J.memo1[kb] = mm;
                     }
@@ -464,9 +459,9 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
             const uint32_t x = x_nx, ok = ok_nx, of = of_nx;
             const float c = c_nx;
             p_nx = p_n2;
-            p_n2 = (base + 64 + lane < e) ? J.ord1[base + 64 + lane] : INT32_MAX;
+            p_n2 = (base + 64 + lane < e) ? cafe_ord(J.ord1, base + 64 + lane) : INT32_MAX;
             x_nx = 0; ok_nx = CAFE_EV_NONE; of_nx = 0; c_nx = 1.0f;
-            if (base + 32 + lane < e) { x_nx = J.sgid1[base + 32 + lane]; if (J.simp1) c_nx = J.simp1[base + 32 + lane]; }
+            if (base + 32 + lane < e) { x_nx = cafe_sid(J.sgid1, base + 32 + lane); if (J.simp1) c_nx = J.simp1[base + 32 + lane]; }
             if (p_nx < J.limit) { ok_nx = cafe_old_kind(J, p_nx); of_nx = cafe_old_mflag(J, p_nx); if (J.final_pass) of_nx |= (uint32_t)J.lflag[p_nx] << 8; }
             const int n = min(32, e - base);
             // Whole chunk = 32 more lookups of the id the previous step dealt with, whose slot owns a hot
@@ -510,7 +505,7 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                 __syncwarp();
                 calm_streak = calm ? streak_in + 1 : 0;
                 if (calm && calm_streak >= 2 && ((base + 32 - s) & 255) == 0 && base + 32 + 511 < e) {
-                    far_at = base + 32; far_x = J.sgid1[far_at + 511]; far_p = J.ord1[far_at + 511];
+                    far_at = base + 32; far_x = cafe_sid(J.sgid1, far_at + 511); far_p = cafe_ord(J.ord1, far_at + 511);
                 }
                 if (lane == o) {
 #pragma unroll
@@ -523,7 +518,7 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                     if (nf != of) J.mflag[p] = (uint8_t)nf;
                     if (!J.first_round) {
                         if (ok != CAFE_EV_NONE) cafe_withdraw_event(J, p);
-                        if (of & CAFE_F_MISS) { J.mark2[cafe_hash(x, J.n2)] = 1; J.res->miss_changed = 1; }
+                        if (of & CAFE_F_MISS) { J.mark2[cafe_hash(x, J.mod2)] = 1; J.res->miss_changed = 1; }
                     }
                 }
                 continue;
@@ -635,12 +630,12 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                             if (nf != of) J.mflag[p] = (uint8_t)nf;
                             if (!J.first_round) {
                                 if (ok != CAFE_EV_NONE) cafe_withdraw_event(J, p);
-                                if (of & CAFE_F_MISS) { J.mark2[cafe_hash(x, J.n2)] = 1; J.res->miss_changed = 1; }
+                                if (of & CAFE_F_MISS) { J.mark2[cafe_hash(x, J.mod2)] = 1; J.res->miss_changed = 1; }
                             }
                         }
                         if (!J.final_pass && in_done && ms < 0) {   // goes to the LRU stage; that pass writes lflag
                             if (of != CAFE_F_MISS) J.mflag[p] = CAFE_F_MISS;
-                            if (!J.first_round && !(of & CAFE_F_MISS)) { J.mark2[cafe_hash(x, J.n2)] = 1; J.res->miss_changed = 1; }   // new visitor
+                            if (!J.first_round && !(of & CAFE_F_MISS)) { J.mark2[cafe_hash(x, J.mod2)] = 1; J.res->miss_changed = 1; }   // new visitor
                         }
                         if (done < run) hvalid = false;
                         j += done;
@@ -1016,7 +1011,7 @@ __device__ __forceinline__ void cafe_lru_body(const CafeJob& J, const CafeHot& H
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 pq[q] = INT32_MAX; xq[q] = 0; cq[q] = 1.0f;
-                if (j + q < jend) { pq[q] = J.ord2[j + q]; xq[q] = J.sgid2[j + q]; if (J.simp2) cq[q] = J.simp2[j + q]; }
+                if (j + q < jend) { pq[q] = cafe_ord(J.ord2, j + q); xq[q] = cafe_sid(J.sgid2, j + q); if (J.simp2) cq[q] = J.simp2[j + q]; }
             }
 #pragma unroll
             for (int q = 0; q < 8; ++q) fq[q] = (pq[q] < J.limit) ? (uint32_t)J.mflag[pq[q]] : 0u;
@@ -1052,9 +1047,9 @@ __device__ __forceinline__ void cafe_lru_body(const CafeJob& J, const CafeHot& H
 #pragma unroll
         for (int q = 0; q < GL; ++q) {
             const int i0 = s + 32 * q + lane, i1 = i0 + 32 * GL, i2 = i1 + 32 * GL;
-            p0[q] = i0 < e ? J.ord2[i0] : INT32_MAX;
-            p1[q] = i1 < e ? J.ord2[i1] : INT32_MAX;
-            p2[q] = i2 < e ? J.ord2[i2] : INT32_MAX;
+            p0[q] = i0 < e ? cafe_ord(J.ord2, i0) : INT32_MAX;
+            p1[q] = i1 < e ? cafe_ord(J.ord2, i1) : INT32_MAX;
+            p2[q] = i2 < e ? cafe_ord(J.ord2, i2) : INT32_MAX;
         }
 #pragma unroll
         for (int q = 0; q < GL; ++q) {
@@ -1065,7 +1060,7 @@ __device__ __forceinline__ void cafe_lru_body(const CafeJob& J, const CafeHot& H
         for (int q = 0; q < GL; ++q) {
             x0[q] = 0; c0[q] = 1.0f; k0[q] = CAFE_EV_NONE;
             if (f0[q] & CAFE_F_MISS) {
-                x0[q] = J.sgid2[s + 32 * q + lane]; if (J.simp2) c0[q] = J.simp2[s + 32 * q + lane];
+                x0[q] = cafe_sid(J.sgid2, s + 32 * q + lane); if (J.simp2) c0[q] = J.simp2[s + 32 * q + lane];
                 if (!J.first_round) k0[q] = J.ev[p0[q]].kind;
             }
         }
@@ -1073,12 +1068,12 @@ __device__ __forceinline__ void cafe_lru_body(const CafeJob& J, const CafeHot& H
 #pragma unroll
             for (int q = 0; q < GL; ++q) {
                 const int i3 = base + 3 * 32 * GL + 32 * q + lane;
-                p3[q] = i3 < e ? J.ord2[i3] : INT32_MAX;
+                p3[q] = i3 < e ? cafe_ord(J.ord2, i3) : INT32_MAX;
                 f2[q] = p2[q] < J.limit ? (uint32_t)J.mflag[p2[q]] : 0u;
                 x1[q] = 0; c1[q] = 1.0f; k1[q] = CAFE_EV_NONE;
                 if (f1[q] & CAFE_F_MISS) {   // (p1 was read at this index of the sorted order)
                     const int i1 = base + 32 * GL + 32 * q + lane;
-                    x1[q] = J.sgid2[i1]; if (J.simp2) c1[q] = J.simp2[i1];
+                    x1[q] = cafe_sid(J.sgid2, i1); if (J.simp2) c1[q] = J.simp2[i1];
                     if (!J.first_round) k1[q] = J.ev[p1[q]].kind;
                 }
             }
@@ -1388,7 +1383,7 @@ struct CafeMissList {
     int32_t* blk;    // [blocks] misses per block of CAFE_TL_BLOCK sorted entries
 };
 __device__ __forceinline__ int cafe_entry_missed(const CafeJob& J, int i) {
-    const int p = J.ord2[i];
+    const int p = cafe_ord(J.ord2, i);
     return (p >= J.begin && p < J.limit && (J.mflag[p] & CAFE_F_MISS)) ? 1 : 0;
 }
 // (a later round in which no lookup entered or left the LRU stage keeps the lists of the round before)
@@ -1441,7 +1436,7 @@ __global__ void __launch_bounds__(128) k_lru_pass_compact(const __grid_constant_
         CafeEvent e_nx; e_nx.x = 0; e_nx.cnt = 0.f; e_nx.dic = 0; e_nx.kind = CAFE_EV_NONE;
         if (jb + lane < jend) {
             const int i = L.list[jb + lane];
-            p_nx = J.ord2[i]; x_nx = J.sgid2[i]; if (J.simp2) c_nx = J.simp2[i];
+            p_nx = cafe_ord(J.ord2, i); x_nx = cafe_sid(J.sgid2, i); if (J.simp2) c_nx = J.simp2[i];
             if (!J.first_round) { e_nx = J.ev[p_nx]; i_nx = J.ins_res[p_nx]; }
         }
         for (int base = jb; base < jend; base += 32) {
@@ -1449,7 +1444,7 @@ __global__ void __launch_bounds__(128) k_lru_pass_compact(const __grid_constant_
             c_nx = 1.0f;
             if (base + 32 + lane < jend) {
                 const int i = L.list[base + 32 + lane];
-                p_nx = J.ord2[i]; x_nx = J.sgid2[i]; if (J.simp2) c_nx = J.simp2[i];
+                p_nx = cafe_ord(J.ord2, i); x_nx = cafe_sid(J.sgid2, i); if (J.simp2) c_nx = J.simp2[i];
                 if (!J.first_round) { e_nx = J.ev[p_nx]; i_nx = J.ins_res[p_nx]; }
             }
             const int n = min(32, jend - base);
@@ -1564,19 +1559,16 @@ struct CudaBackend {
     cudaError_t err = cudaSuccess;
     void* cub_tmp = nullptr;
     size_t cub_bytes = 0;
-    // lane 0 sorts on `stream`; lanes 1 and 2 on side streams with buffers of their own, forked from
-    // and joined to `stream`
-    static const int LANES = 3;
-    // per lane: scratch of the radix sort, intermediate pairs, sorted keys
-    int32_t* sort_scratch[LANES] = {nullptr, nullptr, nullptr};
-    uint32_t *key_tmp[LANES] = {nullptr, nullptr, nullptr}, *key_out[LANES] = {nullptr, nullptr, nullptr};
-    int32_t* pos_tmp[LANES] = {nullptr, nullptr, nullptr};
-    const uint32_t* given_key[LANES] = {nullptr, nullptr, nullptr};   // bucket numbers the caller already has (else hashed here)
+    // the sorts of a call (lookups by main bucket, by LRU bucket, and whatever the caller adds) go in one batch, on
+    // `stream` or on a side stream forked from and joined to it
+    CafeSortBatch batch;                                      // collected so far
+    int32_t* sort_scratch[2] = {nullptr, nullptr};            // per table: scratch of the radix sort, pairs between passes
+    uint2* sort_tmp[2] = {nullptr, nullptr};
     CafeMissList miss = {nullptr, nullptr, nullptr};   // compacted misses of the LRU pass (small sketch, large calls)
     CafeCalmMemo* memo1 = nullptr;   // [n1] last long calm stretch of every main bucket (see the list launch of the main pass)
-    cudaStream_t side[LANES] = {nullptr, nullptr, nullptr};
-    cudaEvent_t ev_fork[LANES] = {nullptr, nullptr, nullptr}, ev_join[LANES] = {nullptr, nullptr, nullptr};
-    bool side_pending[LANES] = {false, false, false};
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    bool side_pending = false;
     int64_t* scan64 = nullptr;   // [4*(n1+n2)] prefix sums of the threshold re-fit
     int32_t* hot_list[2] = {nullptr, nullptr};   // listed long buckets of the main / LRU table
     int32_t* hot_count[2] = {nullptr, nullptr};
@@ -1590,21 +1582,20 @@ struct CudaBackend {
         if (pass_side) { cudaStreamSynchronize(pass_side); cudaStreamDestroy(pass_side); }
         if (pass_ev_fork) cudaEventDestroy(pass_ev_fork);
         if (pass_ev_join) cudaEventDestroy(pass_ev_join);
-        for (int i = 0; i < LANES; ++i) {
-            if (side[i]) { cudaStreamSynchronize(side[i]); cudaStreamDestroy(side[i]); }
-            if (ev_fork[i]) cudaEventDestroy(ev_fork[i]);
-            if (ev_join[i]) cudaEventDestroy(ev_join[i]);
+        if (side) { cudaStreamSynchronize(side); cudaStreamDestroy(side); }
+        if (ev_fork) cudaEventDestroy(ev_fork);
+        if (ev_join) cudaEventDestroy(ev_join);
+        for (int i = 0; i < 2; ++i) {
             if (sort_scratch[i]) cudaFree(sort_scratch[i]);
-            if (key_tmp[i]) cudaFree(key_tmp[i]);
-            if (key_out[i]) cudaFree(key_out[i]);
-            if (pos_tmp[i]) cudaFree(pos_tmp[i]);
+            if (sort_tmp[i]) cudaFree(sort_tmp[i]);
         }
         if (scan64) cudaFree(scan64);
         if (memo1) cudaFree(memo1);
         if (miss.pre) cudaFree(miss.pre);
         if (miss.list) cudaFree(miss.list);
         if (miss.blk) cudaFree(miss.blk);
-        for (int i = 0; i < 2; ++i) { if (hot_list[i]) cudaFree(hot_list[i]); if (hot_count[i]) cudaFree(hot_count[i]); if (hot_flag[i]) cudaFree(hot_flag[i]); }
+        for (int i = 0; i < 2; ++i) { if (hot_list[i]) cudaFree(hot_list[i]); if (hot_flag[i]) cudaFree(hot_flag[i]); }
+        if (hot_count[0]) cudaFree(hot_count[0]);
         if (pinned) cudaFreeHost(pinned);
     }
     void check(cudaError_t e) { if (e != cudaSuccess && err == cudaSuccess) err = e; }
@@ -1662,20 +1653,18 @@ struct CudaBackend {
 
     bool prepare(int cap_, int n1, int n2) {
         cap = cap_;
-        for (int i = 0; i < LANES; ++i) {
-            check(cudaMalloc(&key_tmp[i], 4 * (size_t)cap));
-            check(cudaMalloc(&key_out[i], 4 * (size_t)cap));
-            check(cudaMalloc(&pos_tmp[i], 4 * (size_t)cap));
-            check(cudaMalloc(&sort_scratch[i], 4 * cafe_rs_scratch_elems(cap)));
-            if (i == 0) continue;
-            // (highest priority: the sorts are chains of small kernels that run beside streaming kernels filling every
-            // SM; their blocks must not queue behind those)
-            int lo = 0, hi = 0;
-            check(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-            check(cudaStreamCreateWithPriority(&side[i], cudaStreamNonBlocking, hi));
-            check(cudaEventCreateWithFlags(&ev_fork[i], cudaEventDisableTiming));
-            check(cudaEventCreateWithFlags(&ev_join[i], cudaEventDisableTiming));
+        batch.count = 0;
+        for (int i = 0; i < 2; ++i) {
+            check(cudaMalloc(&sort_tmp[i], sizeof(uint2) * (size_t)cap));
+            check(cudaMalloc(&sort_scratch[i], 4 * cafe_rs_scratch_elems()));
         }
+        // (highest priority: the sorts are chains of small steps that run beside streaming kernels filling every SM;
+        // their blocks must not queue behind those)
+        int lo = 0, hi = 0;
+        check(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+        check(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, hi));
+        check(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+        check(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
         check(cudaMallocHost(&pinned, 4096));
         hot_nb[0] = n1; hot_nb[1] = n2;
         check(cudaMalloc(&miss.pre, 4 * ((size_t)cap + 1)));
@@ -1683,11 +1672,12 @@ struct CudaBackend {
         check(cudaMalloc(&miss.blk, 4 * ((size_t)cap / CAFE_TL_BLOCK + 2)));
         check(cudaMalloc(&memo1, sizeof(CafeCalmMemo) * (size_t)n1));
         check(cudaMemsetAsync(memo1, 0, sizeof(CafeCalmMemo) * (size_t)n1, stream));
+        check(cudaMalloc(&hot_count[0], 16));
+        hot_count[1] = hot_count[0] + 2;
+        check(cudaMemsetAsync(hot_count[0], 0, 16, stream));
         for (int i = 0; i < 2; ++i) {
             check(cudaMalloc(&hot_list[i], 4 * ((size_t)CAFE_HOT_CAP + (size_t)hot_nb[i])));
-            check(cudaMalloc(&hot_count[i], 8));
             check(cudaMalloc(&hot_flag[i], (size_t)hot_nb[i]));
-            check(cudaMemsetAsync(hot_count[i], 0, 8, stream));
             check(cudaMemsetAsync(hot_flag[i], 0, (size_t)hot_nb[i], stream));
         }
         // largest temporary any CUB call below can ask for
@@ -1707,64 +1697,64 @@ struct CudaBackend {
 
     void query(const CafeMainBucket* mb, int n1, const uint32_t* gid, int n, int32_t* out) {
         CAFE_PROF(CAFE_P_QUERY, stream);
-        k_query<<<cafe_blocks(n), CAFE_TPB, 0, stream>>>(mb, n1, gid, n, out);
+        k_query<<<cafe_blocks(n), CAFE_TPB, 0, stream>>>(mb, cafe_mod_of(n1), gid, n, out);
         check_launch();
     }
     void post_query(const CafeMainBucket* mb, int n1, const uint32_t* gid, int n, const int32_t* mask, int32_t* out) {
         CAFE_PROF(CAFE_P_QUERY, stream);
-        k_post_query<<<cafe_blocks(n), CAFE_TPB, 0, stream>>>(mb, n1, gid, n, mask, out);
+        k_post_query<<<cafe_blocks(n), CAFE_TPB, 0, stream>>>(mb, cafe_mod_of(n1), gid, n, mask, out);
         check_launch();
     }
-    static int bits_for(int nb) { int b = 1; while ((1ll << b) < nb) ++b; return b; }
-
-    // positions ordered by (bucket, position): stable LSD radix sort of the bucket index
+    // Positions ordered by (bucket, position), the ids in that order and the buckets' ranges.  The engine asks for the
+    // LRU table's order first (lane 2: only noted) and then for the main table's, which starts both and whatever the
+    // caller added to the batch: lane 0 on `stream`, lane 1 on the side stream.
     void sort_lookups(const uint32_t* gid, int M, int nb, int32_t* ord, uint32_t* sgid, int32_t* start, int32_t* beg, int lane) {
-        cudaStream_t st = stream;
-        if (lane != 0 && cafe_prof_serialise()) lane = -lane;   // the lane's buffers, the caller's stream
-        if (lane > 0) {
-            check(cudaEventRecord(ev_fork[lane], stream));
-            check(cudaStreamWaitEvent(side[lane], ev_fork[lane], 0));
-            st = side[lane];
-        }
-        const bool aside = lane > 0;
-        lane = lane < 0 ? -lane : lane;
-        {
-        CAFE_PROF(CAFE_P_LOOKUP_SORT, st);
-        // the keys are the hashes of the ids (computed in the first pass); the last pass also writes the ids in sorted order
-        CafeKeySource src;
-        src.key = given_key[lane]; src.gid = gid; src.nb = nb;
-        check(cafe_radix_sort(src, nullptr, key_tmp[lane], pos_tmp[lane], key_out[lane], ord, M, bits_for(nb), sort_scratch[lane],
-                              gid, sgid, st));
-        const int t = (nb == hot_nb[0]) ? 0 : 1;
-        k_bucket_starts<<<cafe_blocks((int64_t)M + 1), CAFE_TPB, 0, st>>>(key_out[lane], M, nb, start, hot_count[t]);
-        check_launch();
+        const int t = lane == 2 ? 1 : 0;
+        CafeSortDesc& D = batch.d[batch.count++];
+        (void)ord;   // (the positions lie beside the ids)
+        D.in = gid; D.hashed = 1; D.mod = cafe_mod_of(nb); D.n = M; D.tmp = sort_tmp[t]; D.out = reinterpret_cast<uint2*>(sgid);
+        D.start = start; D.scratch = sort_scratch[t];
         // A warp feeding one long bucket leaves 31 lanes idle while it loads, so it pays where that bucket would
         // otherwise be a serial tail of the thread-per-bucket launch: more lookups than a few times the average
         // load -- but never more than 64, beyond which one thread's serial replay is the tail whatever the average
         // (a sketch of a few thousand rows fed 65536-id calls has hundreds of lookups in EVERY bucket).
-        const int hot_len = std::max(CAFE_HOT_LEN, std::min((int)(16.0 * M / nb), 4096));
-        const int long_len = std::max(16, std::min((int)(4.0 * M / nb), 64));
-        k_find_hot<<<cafe_blocks(nb), CAFE_TPB, 0, st>>>(start, nb, hot_len, long_len, nb, hot_list[t], hot_count[t], hot_flag[t],
-                                                         beg);
-        check_launch();
+        CafeFindHot& F = find[t];
+        F.start = start; F.nb = nb; F.list = hot_list[t]; F.count = hot_count[t]; F.flag = hot_flag[t]; F.beg = beg;
+        F.hot_len = std::max(CAFE_HOT_LEN, std::min((int)(16.0 * M / nb), 4096));
+        F.long_len = std::max(16, std::min((int)(4.0 * M / nb), 64));
+        if (t == 1) return;
+        cudaStream_t st = stream;
+        const bool aside = lane == 1 && !cafe_prof_serialise();
+        if (aside) {
+            check(cudaEventRecord(ev_fork, stream));
+            check(cudaStreamWaitEvent(side, ev_fork, 0));
+            st = side;
+        }
+        {
+            CAFE_PROF(CAFE_P_LOOKUP_SORT, st);
+            check(cafe_radix_sort(batch, st));
+            batch.count = 0;
+            check(cudaMemsetAsync(hot_count[0], 0, 16, st));
+            const dim3 grid((unsigned)cafe_blocks(std::max(find[0].nb, find[1].nb)), 2);
+            k_find_hot<<<grid, CAFE_TPB, 0, st>>>(find[0], find[1]);
+            check_launch();
         }
         if (aside) {
-            check(cudaEventRecord(ev_join[lane], side[lane]));
-            side_pending[lane] = true;
+            check(cudaEventRecord(ev_join, side));
+            side_pending = true;
         }
     }
+    CafeFindHot find[2];
     void gather_counts(const float* imp, const int32_t* ord1, const int32_t* ord2, int M, float* simp1, float* simp2) {
         CAFE_PROF(CAFE_P_LOOKUP_SORT, stream);
         k_gather_counts<<<cafe_blocks(M), CAFE_TPB, 0, stream>>>(imp, ord1, ord2, M, simp1, simp2);
         check_launch();
     }
-    // makes `stream` wait for the sorts outstanding on the side lanes (no-op when there are none)
-    void sort_join(int which) {
-        for (int lane = 1; lane < LANES; ++lane) {
-            if (!side_pending[lane] || (which >= 0 && which != lane)) continue;
-            check(cudaStreamWaitEvent(stream, ev_join[lane], 0));
-            side_pending[lane] = false;
-        }
+    // makes `stream` wait for the sorts outstanding on the side stream (no-op when there are none)
+    void sort_join(int) {
+        if (!side_pending) return;
+        check(cudaStreamWaitEvent(stream, ev_join, 0));
+        side_pending = false;
     }
     // the list launch of a pass runs on a high-priority stream beside the thread-per-bucket launch
     cudaStream_t pass_side = nullptr;
@@ -1947,13 +1937,24 @@ int cafe_internal_insert(void* h, const uint32_t* gid, const float* imp, const i
     int rc = H->eng.insert_segments(gid, imp, seg_off, nseg, mask, post_row, mode != CAFE_INSERT_SEQUENTIAL);
     return finish(H, rc, "cafe_sketch_insert");
 }
-void cafe_internal_presort(void* h, const uint32_t* gid, int n, const uint32_t* key1, const uint32_t* key2, cudaStream_t stream) {
+void cafe_internal_presort(void* h, const uint32_t* gid, int n, const CafeSortDesc* also, cudaStream_t stream) {
     CafeHandle* H = (CafeHandle*)h;
     H->eng.be.stream = stream;
-    H->eng.be.given_key[1] = key1;   // consumed by the two sort_lookups calls of presort
-    H->eng.be.given_key[2] = key2;
+    H->eng.be.batch.count = 0;
+    if (also && gid) H->eng.be.batch.d[H->eng.be.batch.count++] = *also;
     H->eng.presort(gid, n);
-    H->eng.be.given_key[1] = H->eng.be.given_key[2] = nullptr;
+    H->eng.be.batch.count = 0;
+}
+int cafe_internal_sort_wait(void* h, cudaStream_t stream) {
+    CudaBackend& be = ((CafeHandle*)h)->eng.be;
+    if (be.side_pending) be.check(cudaStreamWaitEvent(stream, be.ev_join, 0));
+    return finish((CafeHandle*)h, CAFE_OK, "sort wait");
+}
+int cafe_internal_sort_join(void* h, cudaStream_t stream) {
+    CafeHandle* H = (CafeHandle*)h;
+    H->eng.be.stream = stream;
+    H->eng.be.sort_join(-1);
+    return finish(H, CAFE_OK, "sort join");
 }
 void cafe_internal_set_gate(void* h, int seg, cudaEvent_t ev) {
     CafeHandle* H = (CafeHandle*)h;

@@ -76,8 +76,9 @@ public:
         q_head = 0; q_size = lim - 1;
         // workspace of the parallel insert
         size_t M = (size_t)cap;
-        ord1 = (int32_t*)be.alloc(4 * M); ord2 = (int32_t*)be.alloc(4 * M);
-        sgid1 = (uint32_t*)be.alloc(4 * M); sgid2 = (uint32_t*)be.alloc(4 * M);
+        ent1 = (uint32_t*)be.alloc(8 * M); ent2 = (uint32_t*)be.alloc(8 * M);
+        sgid1 = ent1; ord1 = (int32_t*)(ent1 ? ent1 + (CAFE_ORD_STRIDE == 2 ? 1 : M) : nullptr);
+        sgid2 = ent2; ord2 = (int32_t*)(ent2 ? ent2 + (CAFE_ORD_STRIDE == 2 ? 1 : M) : nullptr);
         simp1 = (float*)be.alloc(4 * M); simp2 = (float*)be.alloc(4 * M);
         start1 = (int32_t*)be.alloc(4 * ((size_t)n1 + 1)); start2 = (int32_t*)be.alloc(4 * ((size_t)n2 + 1));
         beg1 = (int32_t*)be.alloc(4 * (size_t)n1); beg2 = (int32_t*)be.alloc(4 * (size_t)n2);
@@ -146,8 +147,8 @@ public:
         presorted_gid = nullptr;
         if (ready) be.sort_join(-1);   // a null gid withdraws an earlier presort
         if (!ready || !gid || n <= 0 || n > cap) return;
-        be.sort_lookups(gid, n, n1, ord1, sgid1, start1, beg1, 1);
         be.sort_lookups(gid, n, n2, ord2, sgid2, start2, beg2, 2);
+        be.sort_lookups(gid, n, n1, ord1, sgid1, start1, beg1, 1);
         presorted_gid = gid; presorted_n = n;
     }
 
@@ -183,8 +184,7 @@ public:
             struct SortJoin { BE& be; ~SortJoin() { be.sort_join(-1); } } sort_join_guard{be};
             if (parallel && mtot > 0 && !(presorted_gid == g && presorted_n == mtot)) {
                 be.sort_join(-1);   // a head start for other arrays may still be writing the orders
-                // the LRU table's order is first needed by the first LRU pass: it is built on a side
-                // lane of the backend while the main table's order and first pass proceed
+                // (the backend may note the first order and build both at the second call)
                 be.sort_lookups(g, mtot, n2, ord2, sgid2, start2, beg2, 2);
                 be.sort_lookups(g, mtot, n1, ord1, sgid1, start1, beg1, 0);
             }
@@ -326,6 +326,7 @@ private:
     uint32_t* ring = nullptr;
     int32_t *ord1 = nullptr, *ord2 = nullptr, *start1 = nullptr, *start2 = nullptr, *beg1 = nullptr, *beg2 = nullptr;
     uint32_t *sgid1 = nullptr, *sgid2 = nullptr;   // ids in the order of ord1 / ord2
+    uint32_t *ent1 = nullptr, *ent2 = nullptr;     // the memory of both: (id, position) pairs, or ids and then positions
     float *simp1 = nullptr, *simp2 = nullptr;      // counts in the order of ord1 / ord2
     CafeEvent* ev = nullptr;
     int32_t* head = nullptr;
@@ -348,7 +349,7 @@ private:
 
     void release() {
         if (!ready && !mainb[0]) return;
-        void* ptrs[] = {mainb[0], mainb[1], lrub[0], lrub[1], ring, sgid1, sgid2, simp1, simp2, ord1, ord2, start1, start2, beg1, beg2, ev, head, nxt, mark_own, mstate, lstate, mark_w1[0], mflag, lflag, tl_slot, tl_info, tl_size, tl_rank, tl_grp, tl_head, pushbuf, tl_blk, tl_agg, nmiss,
+        void* ptrs[] = {mainb[0], mainb[1], lrub[0], lrub[1], ring, ent1, ent2, simp1, simp2, start1, start2, beg1, beg2, ev, head, nxt, mark_own, mstate, lstate, mark_w1[0], mflag, lflag, tl_slot, tl_info, tl_size, tl_rank, tl_grp, tl_head, pushbuf, tl_blk, tl_agg, nmiss,
                         ins_res, seq_dev, cand_key[0], cand_key[1],
                         cand_val[0], cand_val[1], cand_cnt, reset_out};
         for (void* p : ptrs) if (p) be.free(p);
@@ -399,7 +400,7 @@ private:
         for (int i = nseg + 1; i <= CAFE_MAX_SEGMENTS; ++i) J.seg_off[i] = INT32_MAX;
         J.ord1 = ord1; J.start1 = start1; J.beg1 = beg1; J.ord2 = ord2; J.start2 = start2; J.beg2 = beg2;
         J.sgid1 = sgid1; J.sgid2 = sgid2; J.simp1 = imp ? simp1 : nullptr; J.simp2 = imp ? simp2 : nullptr;
-        J.n1 = n1; J.n2 = n2; J.thr = thr; J.gflip = gflip; J.t0 = t;
+        J.n1 = n1; J.n2 = n2; J.mod1 = cafe_mod_of(n1); J.mod2 = cafe_mod_of(n2); J.thr = thr; J.gflip = gflip; J.t0 = t;
         J.ring = ring; J.ring_mask = ring_mask; J.q_head = q_head; J.q_size = q_size;
         J.main_in = mainb[cur]; J.main_out = mainb[cur ^ 1];
         J.lru_in = lrub[cur]; J.lru_out = lrub[cur ^ 1];
