@@ -45,8 +45,9 @@ void cafe_embed_ws_free(CafeEmbedWorkspace* ws);
 
 CafeSketchView cafe_internal_view(void* h);
 CafeEmbedWorkspace* cafe_internal_ws(void* h);
+// use_presort: the last cafe_internal_presort was for exactly these ids (and they have not changed since)
 int cafe_internal_insert(void* h, const uint32_t* gid, const float* imp, const int* seg_off, int nseg, int32_t* mask,
-                         int32_t* post_row, int mode, cudaStream_t stream);
+                         int32_t* post_row, int mode, bool use_presort, cudaStream_t stream);
 // starts the insert's bucket sorts of `gid` beside whatever the caller queues next on `stream`
 // (also: a further sort to run with them, or null).  A null gid withdraws an earlier presort.
 void cafe_internal_presort(void* h, const uint32_t* gid, int n, const CafeSortDesc* also, cudaStream_t stream);

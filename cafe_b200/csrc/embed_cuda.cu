@@ -665,6 +665,14 @@ static bool strides_ok(const float* p, int64_t fs, int64_t ss) { return aligned1
         default: { constexpr int G = 32; CALL; } break; \
     }
 
+// A forward has (re)written these two arrays: a head start or row keys left for arrays at the same addresses (of a
+// forward whose backward never came) belong to other lookups.
+static void forget_head_start(void* h, const uint32_t* gid, const int32_t* row) {
+    CafeEmbedWorkspace* ws = cafe_internal_ws(h);
+    if (ws->begun_gid == gid || ws->begun_row == row) { ws->begun_gid = nullptr; ws->begun_row = nullptr; ws->begun_total = 0; }
+    if (ws->keys_of == gid) ws->keys_of = nullptr;
+}
+
 static int launch_forward(const CafeFields& F, const void* ids_dev, int ids_are_int64, const CafeSketchView& V,
                           const CafeRankBuffers& out_dev, int64_t out_field_stride, int64_t out_sample_stride,
                           uint32_t* gid_out_dev, int32_t* row_out_dev, int total, int D, cudaStream_t st) {
@@ -702,6 +710,7 @@ int cafe_embed_forward(void* h, const void* ids_dev, int ids_are_int64, int nfie
     memset(&ob, 0, sizeof(ob));
     ob.base[0] = out_dev;
     ob.rows_per_rank = B > 0 ? B : 1;
+    forget_head_start(h, gid_out_dev, row_out_dev);
     return launch_forward(F, ids_dev, ids_are_int64, V, ob, out_field_stride, out_sample_stride, gid_out_dev, row_out_dev, total, D, st);
 }
 
@@ -745,6 +754,7 @@ int cafe_embed_resolve(void* h, const void* ids_dev, int ids_are_int64, int nfie
     const bool keep = total <= ws->cap && rows + hotn <= 0x7fffffffLL;
     uint32_t* keys = keep ? ws->key : nullptr;
     const CafeMod mod = cafe_mod_of(V.n1);
+    forget_head_start(h, gid_out_dev, row_out_dev);
     ws->keys_of = keep ? gid_out_dev : nullptr;
     ws->keys_total = keep ? total : 0;
     cudaStream_t st = (cudaStream_t)stream;
@@ -981,14 +991,20 @@ int cafe_scatter_sgd(void* h, const float* grad_dev, int64_t field_stride, int64
 // of the scatter and the bucket sorts of the parallel insert, in one batch on a stream of the sketch's.
 static int backward_side_work(void* h, CafeEmbedWorkspace* ws, const CafeFields& FS, const uint32_t* gid_dev,
                               const int32_t* row_dev, int total, int insert_mode, cudaStream_t st) {
+    // (row keys serve the lookups they were left for once: the arrays may be the caller's to rewrite afterwards)
     const bool begun = ws->begun_gid == gid_dev && ws->begun_row == row_dev && ws->begun_total == total &&
                        ws->begun_mode == insert_mode && gid_dev != nullptr;
     ws->begun_gid = nullptr; ws->begun_row = nullptr; ws->begun_total = 0;
     if (begun) return CAFE_OK;
+    {   // sorts started for other lookups may still be using the arrays
+        const int rc = cafe_internal_sort_wait(h, st);
+        if (rc != CAFE_OK) return rc;
+    }
     if (insert_mode == CAFE_INSERT_SEQUENTIAL) { ws->keys_of = nullptr; return scatter_prepare(ws, FS, row_dev, total, st); }
     // row keys left by cafe_embed_resolve for exactly these lookups
     const bool have = ws->keys_of == gid_dev && ws->keys_total == total;
-    if (!have) { row_keys(ws, FS, row_dev, total, st); ws->keys_of = nullptr; }
+    ws->keys_of = nullptr;
+    if (!have) row_keys(ws, FS, row_dev, total, st);
     const CafeSortDesc rows = row_sort_desc(ws, FS, total);
     cafe_internal_presort(h, gid_dev, total, &rows, st);
     return CAFE_OK;
@@ -1057,7 +1073,7 @@ static int embed_backward_impl(void* h, const float* grad_dev, int64_t field_str
     int seg[CAFE_MAX_SEGMENTS + 1];
     for (int f = 0; f <= nfields; ++f) seg[f] = f * B;
     int32_t* mask = mask_out_dev ? mask_out_dev : ws->mask;
-    int status = cafe_internal_insert(h, gid_dev, ws->imp, seg, nfields, mask, ws->post_row, insert_mode, st);
+    int status = cafe_internal_insert(h, gid_dev, ws->imp, seg, nfields, mask, ws->post_row, insert_mode, true, st);
     cafe_internal_set_gate(h, -1, nullptr);
     if (gated) cudaStreamWaitEvent(st, ws->ev_late, 0);   // whatever the insert did: the scatter reads every field
     rc = cafe_internal_sort_join(h, st);
@@ -1126,6 +1142,7 @@ int cafe_embed_forward_sharded(void* h, const void* ids_dev, int ids_are_int64, 
     ob.rows_per_rank = rows_per_rank;
     CafeSketchView V = cafe_internal_view(h);
     if (hotn != V.lim) return CAFE_ERR_ARG;
+    forget_head_start(h, gid_out_dev, row_out_dev);
     return launch_forward(F, ids_dev, ids_are_int64, V, ob, out_field_stride, out_sample_stride, gid_out_dev, row_out_dev, total, D,
                           (cudaStream_t)stream);
 }
@@ -1194,7 +1211,7 @@ int cafe_embed_backward_imp(void* h, const float* grad_dev, int64_t field_stride
     if (rc != CAFE_OK) return rc;
     rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, insert_mode, (cudaStream_t)stream);
     if (rc != CAFE_OK) return rc;
-    int status = cafe_internal_insert(h, gid_dev, imp_dev, seg, nfields, mask, ws->post_row, insert_mode, (cudaStream_t)stream);
+    int status = cafe_internal_insert(h, gid_dev, imp_dev, seg, nfields, mask, ws->post_row, insert_mode, true, (cudaStream_t)stream);
     rc = cafe_internal_sort_join(h, (cudaStream_t)stream);
     if (status != CAFE_OK && status != CAFE_ERR_NOCONVERGE && status != CAFE_ERR_RESET_UNDERFLOW) return status;
     if (rc != CAFE_OK) return rc;
@@ -1287,7 +1304,7 @@ int cafe_embed_backward_norms(void* h, const float* grad_dev, int64_t field_stri
                                                                                                     (int)total, ws->imp); }
     int seg[CAFE_MAX_SEGMENTS + 1];
     for (int f = 0; f <= nfields; ++f) seg[f] = f * B;
-    int status = cafe_internal_insert(h, gid_dev, ws->imp, seg, nfields, ws->mask, ws->post_row, insert_mode, st);
+    int status = cafe_internal_insert(h, gid_dev, ws->imp, seg, nfields, ws->mask, ws->post_row, insert_mode, true, st);
     rc = cafe_internal_sort_join(h, st);
     if (status != CAFE_OK && status != CAFE_ERR_NOCONVERGE && status != CAFE_ERR_RESET_UNDERFLOW) return status;
     if (rc != CAFE_OK) return rc;

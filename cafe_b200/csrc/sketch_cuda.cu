@@ -1931,9 +1931,10 @@ CafeSketchView cafe_internal_view(void* h) {
 }
 CafeEmbedWorkspace* cafe_internal_ws(void* h) { return &((CafeHandle*)h)->ws; }
 int cafe_internal_insert(void* h, const uint32_t* gid, const float* imp, const int* seg_off, int nseg, int32_t* mask,
-                         int32_t* post_row, int mode, cudaStream_t stream) {
+                         int32_t* post_row, int mode, bool use_presort, cudaStream_t stream) {
     CafeHandle* H = (CafeHandle*)h;
     H->eng.be.stream = stream;
+    if (!use_presort) H->eng.presort(nullptr, 0);
     int rc = H->eng.insert_segments(gid, imp, seg_off, nseg, mask, post_row, mode != CAFE_INSERT_SEQUENTIAL);
     return finish(H, rc, "cafe_sketch_insert");
 }
@@ -2023,7 +2024,7 @@ int cafe_sketch_query(void* h, const uint32_t* gid_dev, int n, int32_t* out_dev,
 int cafe_sketch_insert(void* h, const uint32_t* gid_dev, const float* imp_dev, const int* seg_off_host, int nseg,
                        int32_t* mask_dev, int32_t* post_row_dev, int mode, void* stream) {
     CAFE_H(h);
-    return cafe_internal_insert(h, gid_dev, imp_dev, seg_off_host, nseg, mask_dev, post_row_dev, mode, (cudaStream_t)stream);
+    return cafe_internal_insert(h, gid_dev, imp_dev, seg_off_host, nseg, mask_dev, post_row_dev, mode, false, (cudaStream_t)stream);
 }
 
 int cafe_sketch_refit(void* h, void* stream) {

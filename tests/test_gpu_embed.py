@@ -332,3 +332,40 @@ def test_two_fields_claim_one_hot_row_in_one_step():
         assert states_equal(sk.state(), grp.sketch.state()) == [], f"step {step}"
         close(grp.weight_high.detach().cpu().numpy(), orc.wh, f"step {step}: hot table")
     assert grp.sketch.stats()["resets"] > 0
+
+
+def test_a_dropped_forward_leaves_nothing_behind():
+    """A training forward whose backward never comes (its head start is under way, its buffers are freed), then a forward
+    in eval mode whose buffers the allocator places at the same addresses, and that one's backward: the row order and the
+    bucket orders must be those of the second batch."""
+    import torch
+    import cafe_b200
+    from oracle.hotsketch import OracleSketch, states_equal
+    from oracle.module_oracle import ModuleOracle
+    cards, D, B = [3000, 50000], 16, 300
+    grp = cafe_b200.SKEmbeddingGroup(cards, D, 0.02, 0.3, 1, 1, 1.0000005, device="cuda", max_batch=B, lr=0.1, seed=4)
+    sk = OracleSketch(grp.hotn, 1, 1, 1.0000005)
+    orc = ModuleOracle(sk, grp.weight_high.detach().cpu().numpy(), [w.detach().cpu().numpy() for w in grp.weight_hash],
+                       grp.f_offsets, grp.hash_sizes)
+    rng = np.random.default_rng(8)
+    for step in range(6):
+        dropped = np.stack([rng.integers(0, n, B) for n in cards]).astype(np.int64)
+        ids = np.stack([np.minimum(rng.zipf(1.3, B) - 1, n - 1) for n in cards]).astype(np.int64)
+        grp.train()
+        out = grp(torch.from_numpy(dropped).cuda())
+        del out
+        grp.last_rows = None
+        if step % 2:
+            grp.row_codes(torch.from_numpy(dropped).cuda())
+        grp.eval()
+        out = grp(torch.from_numpy(ids).cuda())
+        orc.forward(ids)
+        grad = (rng.standard_normal((B, 2, D)) * 0.01).astype(np.float32)
+        g = torch.from_numpy(grad).cuda()
+        imp = grp._fields.importance(g, D, 2 * D, B).view(2, B).cpu().numpy()
+        out.backward(g)
+        orc.backward(ids, grad, grp.lr, importance=imp)
+        assert states_equal(sk.state(), grp.sketch.state()) == [], f"step {step}"
+        np.testing.assert_allclose(grp.weight_high.detach().cpu().numpy(), orc.wh, rtol=1e-5, atol=1e-7)
+        for f in range(2):
+            np.testing.assert_allclose(grp.weight_hash[f].detach().cpu().numpy(), orc.wc[f], rtol=1e-5, atol=1e-7)
