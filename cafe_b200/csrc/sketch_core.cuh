@@ -228,6 +228,7 @@ struct alignas(16) CafeFn { int32_t a, b, np, pad; };   // FIFO size transfer s 
 
 // The FIFO timeline is kept sparse: one entry per op (a candidate pop or a push), in op-slot order.
 #define CAFE_TL_BLOCK 1024    // positions (resp. ops) handled by one block of the timeline kernels
+#define CAFE_TL_SMALL 128     // the smallest such block (the scratch is sized for it)
 #define CAFE_TL_GROUP 64      // positions per entry of the coarse index into the op list
 
 #if defined(__CUDACC__)

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdio.h>
 
+#include <cooperative_groups.h>
+
 #include <cub/cub.cuh>
 #include <algorithm>
 #include <string>
@@ -37,20 +39,20 @@ struct CafeFills {
     int v[4];
     int count;
 };
+__device__ __forceinline__ void cafe_fill(void* p_, int v, size_t n, size_t tid, size_t nth) {
+    unsigned char* p = (unsigned char*)p_;
+    const unsigned b = (unsigned)v & 0xffu;
+    const unsigned w = b * 0x01010101u;
+    size_t head = (16 - ((uintptr_t)p & 15)) & 15;
+    if (head > n) head = n;
+    const size_t body = (n - head) / 16, tail0 = head + 16 * body;
+    for (size_t i = tid; i < body; i += nth) reinterpret_cast<uint4*>(p + head)[i] = make_uint4(w, w, w, w);
+    for (size_t i = tid; i < head; i += nth) p[i] = (unsigned char)b;
+    for (size_t i = tail0 + tid; i < n; i += nth) p[i] = (unsigned char)b;
+}
 __global__ void k_fills(const CafeFills F) {
     const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (size_t)gridDim.x * blockDim.x;
-    for (int s = 0; s < F.count; ++s) {
-        unsigned char* p = F.p[s];
-        const size_t n = F.n[s];
-        const unsigned b = (unsigned)F.v[s] & 0xffu;
-        const unsigned w = b * 0x01010101u;
-        size_t head = (16 - ((uintptr_t)p & 15)) & 15;
-        if (head > n) head = n;
-        const size_t body = (n - head) / 16, tail0 = head + 16 * body;
-        for (size_t i = tid; i < body; i += nth) reinterpret_cast<uint4*>(p + head)[i] = make_uint4(w, w, w, w);
-        for (size_t i = tid; i < head; i += nth) p[i] = (unsigned char)b;
-        for (size_t i = tail0 + tid; i < n; i += nth) p[i] = (unsigned char)b;
-    }
+    for (int s = 0; s < F.count; ++s) cafe_fill(F.p[s], F.v[s], F.n[s], tid, nth);
 }
 
 __global__ void k_query(const CafeMainBucket* __restrict__ mb, const CafeMod n1, const uint32_t* __restrict__ gid, int n,
@@ -1178,8 +1180,11 @@ __global__ void k_commit_tables(const __grid_constant__ CafeJob J, int32_t* beg1
 // CAFE_TL_PER consecutive ones per thread, so that a scan over threads is a scan in position order.
 #define CAFE_TL_THREADS 256
 #define CAFE_TL_PER (CAFE_TL_BLOCK / CAFE_TL_THREADS)
+// (the steps are functions of the block size and of the block's number, so that they serve a launch per step and the
+// whole-job kernel below)
 
 // exclusive prefix of v over the block's threads (in thread order) and the block total
+template <int T = CAFE_TL_THREADS>
 __device__ __forceinline__ int cafe_block_exclusive_sum(int v, int* total, int* s_warp) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int inc = v;
@@ -1192,13 +1197,14 @@ __device__ __forceinline__ int cafe_block_exclusive_sum(int v, int* total, int* 
     __syncthreads();
     int before = 0, all = 0;
 #pragma unroll
-    for (int q = 0; q < CAFE_TL_THREADS / 32; ++q) { const int t = s_warp[q]; if (q < w) before += t; all += t; }
+    for (int q = 0; q < T / 32; ++q) { const int t = s_warp[q]; if (q < w) before += t; all += t; }
     __syncthreads();
     *total = all;
     return before + inc - v;
 }
 // the same for the FIFO-size transfer functions (composition is associative but not commutative:
 // earlier entries are always the left operand)
+template <int T = CAFE_TL_THREADS>
 __device__ __forceinline__ CafeFn cafe_block_exclusive_fn(const CafeFn& v, CafeFn* total, CafeFn* s_warp) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     CafeFn inc = v;
@@ -1217,7 +1223,7 @@ __device__ __forceinline__ CafeFn cafe_block_exclusive_fn(const CafeFn& v, CafeF
     __syncthreads();
     CafeFn before = cafe_fn_identity(), all = cafe_fn_identity();
 #pragma unroll
-    for (int q = 0; q < CAFE_TL_THREADS / 32; ++q) {
+    for (int q = 0; q < T / 32; ++q) {
         const CafeFn t = s_warp[q];
         if (q < w) before = cafe_fn_then(before, t);
         all = cafe_fn_then(all, t);
@@ -1230,19 +1236,20 @@ __device__ __forceinline__ CafeFn cafe_block_exclusive_fn(const CafeFn& v, CafeF
 // 3a, first half: ops and main-table misses per block of positions; per-segment threshold crossings and the
 // number of LRU visits as block-wide sums, one atomic per block and counter (a block of consecutive
 // positions lies in one segment except at boundaries)
-__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_count(const __grid_constant__ CafeJob J) {
-    __shared__ int s_warp[CAFE_TL_THREADS / 32];
-    __shared__ int s_cross;
-    const int first = J.begin + blockIdx.x * CAFE_TL_BLOCK;
-    const int last = min(first + CAFE_TL_BLOCK, J.limit) - 1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) J.tl_blk[2 * gridDim.x] = J.tl_head[0];   // the old list's length, for k_tl_emit
+template <int T, int PER>
+__device__ __forceinline__ void cafe_tl_count_block(const CafeJob& J, const int blk, const int nblk, int* s_warp, int* s_cross_p) {
+    constexpr int BLOCK = T * PER;
+    int& s_cross = *s_cross_p;
+    const int first = J.begin + blk * BLOCK;
+    const int last = min(first + BLOCK, J.limit) - 1;
+    if (blk == 0 && threadIdx.x == 0) J.tl_blk[2 * nblk] = J.tl_head[0];   // the old list's length, for the emit step
     if (threadIdx.x == 0) s_cross = 0;
     __syncthreads();
     const int seg_first = cafe_segment_of(J, first), seg_last = cafe_segment_of(J, last);
     int ops = 0, miss = 0, cross = 0;
 #pragma unroll
-    for (int i = 0; i < CAFE_TL_PER; ++i) {
-        const int p = first + threadIdx.x * CAFE_TL_PER + i;
+    for (int i = 0; i < PER; ++i) {
+        const int p = first + threadIdx.x * PER + i;
         if (p >= J.limit) break;
         ops += cafe_ops_count(cafe_ops_of(J, p));
         int c, mi;
@@ -1251,98 +1258,118 @@ __global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_count(const __grid_const
         if (c) { if (seg_first == seg_last) ++cross; else atomicAdd(&J.res->seg_real_delta[cafe_segment_of(J, p)], 1); }
     }
     int tot_ops, tot_miss;
-    cafe_block_exclusive_sum(ops, &tot_ops, s_warp);
-    cafe_block_exclusive_sum(miss, &tot_miss, s_warp);
+    cafe_block_exclusive_sum<T>(ops, &tot_ops, s_warp);
+    cafe_block_exclusive_sum<T>(miss, &tot_miss, s_warp);
     if (cross) atomicAdd(&s_cross, cross);
     __syncthreads();
     if (threadIdx.x == 0) {
-        J.tl_blk[2 * blockIdx.x] = tot_ops;
-        J.tl_blk[2 * blockIdx.x + 1] = tot_miss;
+        J.tl_blk[2 * blk] = tot_ops;
+        J.tl_blk[2 * blk + 1] = tot_miss;
         if (s_cross) atomicAdd(&J.res->seg_real_delta[seg_first], s_cross);
         if (tot_miss) atomicAdd(&J.res->n_miss, tot_miss);
     }
 }
+__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_count(const __grid_constant__ CafeJob J) {
+    __shared__ int s_warp[CAFE_TL_THREADS / 32];
+    __shared__ int s_cross;
+    cafe_tl_count_block<CAFE_TL_THREADS, CAFE_TL_PER>(J, blockIdx.x, gridDim.x, s_warp, &s_cross);
+}
 // sum of the per-block counts (kind 0: ops, 1: misses) of the blocks ahead of this one
-__device__ __forceinline__ int cafe_tl_blocks_before(const CafeJob& J, int kind, int* s_warp) {
+template <int T>
+__device__ __forceinline__ int cafe_tl_blocks_before(const CafeJob& J, const int blk, int kind, int* s_warp) {
     int v = 0;
-    for (int q = threadIdx.x; q < (int)blockIdx.x; q += CAFE_TL_THREADS) v += J.tl_blk[2 * q + kind];
+    for (int q = threadIdx.x; q < blk; q += T) v += J.tl_blk[2 * q + kind];
     int tot;
-    cafe_block_exclusive_sum(v, &tot, s_warp);
+    cafe_block_exclusive_sum<T>(v, &tot, s_warp);
     return tot;
 }
 // 3a, second half: the ops go to their places in the list (updated in place, compared with the old entries)
-__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_emit(const __grid_constant__ CafeJob J) {
-    __shared__ int s_warp[CAFE_TL_THREADS / 32];
-    const int first = J.begin + blockIdx.x * CAFE_TL_BLOCK;
-    const int32_t n_old = J.tl_blk[2 * gridDim.x];
-    const int base = cafe_tl_blocks_before(J, 0, s_warp);
-    CafeOps o[CAFE_TL_PER];
+template <int T, int PER>
+__device__ __forceinline__ void cafe_tl_emit_block(const CafeJob& J, const int blk, const int nblk, int* s_warp) {
+    constexpr int BLOCK = T * PER;
+    const int first = J.begin + blk * BLOCK;
+    const int32_t n_old = J.tl_blk[2 * nblk];
+    const int base = cafe_tl_blocks_before<T>(J, blk, 0, s_warp);
+    CafeOps o[PER];
     int cnt = 0;
 #pragma unroll
-    for (int i = 0; i < CAFE_TL_PER; ++i) {
-        const int p = first + threadIdx.x * CAFE_TL_PER + i;
+    for (int i = 0; i < PER; ++i) {
+        const int p = first + threadIdx.x * PER + i;
         o[i].op0 = o[i].op1 = 0;
         if (p < J.limit) { o[i] = cafe_ops_of(J, p); cnt += cafe_ops_count(o[i]); }
     }
     int tot;
-    int j = base + cafe_block_exclusive_sum(cnt, &tot, s_warp);
-    const int p0 = first + threadIdx.x * CAFE_TL_PER;
+    int j = base + cafe_block_exclusive_sum<T>(cnt, &tot, s_warp);
+    const int p0 = first + threadIdx.x * PER;
     if (p0 < J.limit && (p0 - J.begin) % CAFE_TL_GROUP == 0) J.tl_grp[(p0 - J.begin) / CAFE_TL_GROUP] = j;
 #pragma unroll
-    for (int i = 0; i < CAFE_TL_PER; ++i) {
+    for (int i = 0; i < PER; ++i) {
         const int p = p0 + i;
         if (p >= J.limit) break;
         cafe_tl_emit(J, p, o[i], j, n_old);
         j += cafe_ops_count(o[i]);
     }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    if (blk == nblk - 1 && threadIdx.x == 0) {
         J.tl_grp[(J.limit - J.begin + CAFE_TL_GROUP - 1) / CAFE_TL_GROUP] = base + tot;
         cafe_tl_set_count(J, base + tot, n_old);
     }
 }
+__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_emit(const __grid_constant__ CafeJob J) {
+    __shared__ int s_warp[CAFE_TL_THREADS / 32];
+    cafe_tl_emit_block<CAFE_TL_THREADS, CAFE_TL_PER>(J, blockIdx.x, gridDim.x, s_warp);
+}
 // 3b, first half: composed transfer function of every block of list entries (the list is usually short: a
 // fixed small grid walks over its blocks)
-__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_aggregate(const __grid_constant__ CafeJob J) {
-    __shared__ CafeFn s_warp[CAFE_TL_THREADS / 32];
+template <int T, int PER>
+__device__ __forceinline__ void cafe_tl_aggregate_blocks(const CafeJob& J, CafeFn* s_warp) {
+    constexpr int BLOCK = T * PER;
     const int32_t n = J.tl_head[0];
-    for (int blk = blockIdx.x; blk * CAFE_TL_BLOCK < n; blk += gridDim.x) {
-        const int base = blk * CAFE_TL_BLOCK;
+    for (int blk = blockIdx.x; blk * BLOCK < n; blk += gridDim.x) {
+        const int base = blk * BLOCK;
         CafeFn v = cafe_fn_identity();
 #pragma unroll
-        for (int i = 0; i < CAFE_TL_PER; ++i) {
-            const int j = base + threadIdx.x * CAFE_TL_PER + i;
+        for (int i = 0; i < PER; ++i) {
+            const int j = base + threadIdx.x * PER + i;
             if (j < n) v = cafe_fn_then(v, cafe_fn_of_info(J.tl_info[j]));
         }
         CafeFn tot;
-        cafe_block_exclusive_fn(v, &tot, s_warp);
+        cafe_block_exclusive_fn<T>(v, &tot, s_warp);
         if (threadIdx.x == 0) J.tl_agg[blk] = tot;
     }
 }
-// 3b, second half: FIFO size and successful pops before every list entry, the pushed rows in order, totals
-__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_finish(const __grid_constant__ CafeJob J) {
+__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_aggregate(const __grid_constant__ CafeJob J) {
     __shared__ CafeFn s_warp[CAFE_TL_THREADS / 32];
-    __shared__ CafeFn s_before;
+    cafe_tl_aggregate_blocks<CAFE_TL_THREADS, CAFE_TL_PER>(J, s_warp);
+}
+// 3b, second half: FIFO size and successful pops before every list entry, the pushed rows in order, totals
+// (the blocks ahead are composed by the block's threads, each taking consecutive ones)
+template <int T, int PER>
+__device__ __forceinline__ void cafe_tl_finish_blocks(const CafeJob& J, CafeFn* s_warp, CafeFn* s_before_p) {
+    constexpr int BLOCK = T * PER;
+    CafeFn& s_before = *s_before_p;
     const int32_t n = J.tl_head[0];
-    for (int blk = blockIdx.x; blk * CAFE_TL_BLOCK < n; blk += gridDim.x) {
-        const int base = blk * CAFE_TL_BLOCK;
-        if (threadIdx.x == 0) {
-            CafeFn f = cafe_fn_identity();
-            for (int q = 0; q < blk; ++q) f = cafe_fn_then(f, J.tl_agg[q]);
-            s_before = f;
+    for (int blk = blockIdx.x; blk * BLOCK < n; blk += gridDim.x) {
+        const int base = blk * BLOCK;
+        {
+            CafeFn f = cafe_fn_identity(), all;
+            const int each = (blk + T - 1) / T;
+            for (int q = threadIdx.x * each; q < min(blk, ((int)threadIdx.x + 1) * each); ++q) f = cafe_fn_then(f, J.tl_agg[q]);
+            cafe_block_exclusive_fn<T>(f, &all, s_warp);
+            if (threadIdx.x == 0) s_before = all;
         }
         __syncthreads();
-        const int j0 = base + threadIdx.x * CAFE_TL_PER;
+        const int j0 = base + threadIdx.x * PER;
         CafeFn v = cafe_fn_identity();
-        int32_t info[CAFE_TL_PER];
+        int32_t info[PER];
 #pragma unroll
-        for (int i = 0; i < CAFE_TL_PER; ++i) {
+        for (int i = 0; i < PER; ++i) {
             info[i] = (j0 + i < n) ? J.tl_info[j0 + i] : 0;
             if (j0 + i < n) v = cafe_fn_then(v, cafe_fn_of_info(info[i]));
         }
         CafeFn tot;
-        CafeFn before = cafe_fn_then(s_before, cafe_block_exclusive_fn(v, &tot, s_warp));
+        CafeFn before = cafe_fn_then(s_before, cafe_block_exclusive_fn<T>(v, &tot, s_warp));
 #pragma unroll
-        for (int i = 0; i < CAFE_TL_PER; ++i) {
+        for (int i = 0; i < PER; ++i) {
             if (j0 + i >= n) break;
             cafe_tl_finish_op(J, j0 + i, n, before);
             before = cafe_fn_then(before, cafe_fn_of_info(info[i]));
@@ -1350,26 +1377,36 @@ __global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_finish(const __grid_cons
         __syncthreads();
     }
 }
+__global__ void __launch_bounds__(CAFE_TL_THREADS) k_tl_finish(const __grid_constant__ CafeJob J) {
+    __shared__ CafeFn s_warp[CAFE_TL_THREADS / 32];
+    __shared__ CafeFn s_before;
+    cafe_tl_finish_blocks<CAFE_TL_THREADS, CAFE_TL_PER>(J, s_warp, &s_before);
+}
 // at commit: main-table misses up to and including every position of the job (the LRU clock numbering)
-__global__ void __launch_bounds__(CAFE_TL_THREADS) k_miss_prefix(const __grid_constant__ CafeJob J) {
-    __shared__ int s_warp[CAFE_TL_THREADS / 32];
-    const int first = J.begin + blockIdx.x * CAFE_TL_BLOCK;
-    const int base = cafe_tl_blocks_before(J, 1, s_warp);
-    const int p0 = first + threadIdx.x * CAFE_TL_PER;
-    int m[CAFE_TL_PER], cnt = 0;
+template <int T, int PER>
+__device__ __forceinline__ void cafe_miss_prefix_block(const CafeJob& J, const int blk, int* s_warp) {
+    constexpr int BLOCK = T * PER;
+    const int first = J.begin + blk * BLOCK;
+    const int base = cafe_tl_blocks_before<T>(J, blk, 1, s_warp);
+    const int p0 = first + threadIdx.x * PER;
+    int m[PER], cnt = 0;
 #pragma unroll
-    for (int i = 0; i < CAFE_TL_PER; ++i) {
+    for (int i = 0; i < PER; ++i) {
         m[i] = (p0 + i < J.limit && (J.mflag[p0 + i] & CAFE_F_MISS)) ? 1 : 0;
         cnt += m[i];
     }
     int tot;
-    int run = base + cafe_block_exclusive_sum(cnt, &tot, s_warp);
+    int run = base + cafe_block_exclusive_sum<T>(cnt, &tot, s_warp);
 #pragma unroll
-    for (int i = 0; i < CAFE_TL_PER; ++i) {
+    for (int i = 0; i < PER; ++i) {
         if (p0 + i >= J.limit) break;
         run += m[i];
         J.nmiss[p0 + i] = run;
     }
+}
+__global__ void __launch_bounds__(CAFE_TL_THREADS) k_miss_prefix(const __grid_constant__ CafeJob J) {
+    __shared__ int s_warp[CAFE_TL_THREADS / 32];
+    cafe_miss_prefix_block<CAFE_TL_THREADS, CAFE_TL_PER>(J, blockIdx.x, s_warp);
 }
 // ---- LRU pass over compacted miss lists --------------------------------------------------------------
 // When a small sketch is fed large calls, an LRU bucket's sorted stretch holds thousands of lookups of which
@@ -1453,6 +1490,197 @@ __global__ void __launch_bounds__(128) k_lru_pass_compact(const __grid_constant_
         }
         if (lane == 0) R.finish(J);
     }
+}
+// ---- a whole job in one launch ----------------------------------------------------------------------------------------
+// A round is eight or nine steps of microseconds each, and a job has three to six rounds.  Launched one by one with a
+// read-back per round they are nearly all launch gaps and waits of the host.  So jobs that a resident grid can carry run
+// in ONE cooperative launch: the steps are separated by the grid's barrier, every block takes the round's decision (go on,
+// shorten the job at a re-fit, finish) from the round result itself, and the host reads one record at the end.  The
+// steps are the functions of the launches above; the job lives in shared memory because rounds and shortenings change it.
+//
+// What bounds it is the chain of dependent loads of every step and the slowest bucket of a pass; a barrier takes 1.2 us.  A
+// step's insert of 26 x 128 lookups (12 000 buckets) takes 91 us of it, of 26 x 2048 (108 000 buckets) 147 us, of 9 x 4096
+// (146 000 buckets) 149 us.  Training steps against the launches: Kaggle shape 441 -> 363 us, Terabyte 510 -> 464, Avazu
+// 408 -> 346, 11 x 777 342 -> 313, four modules of 2048 1253 -> 1144.
+#define CAFE_JOB_THREADS 128
+// Beyond this many lookups the passes are bound by their work and want the launches' occupancy (24 warps per SM against 12
+// here, and a launch of their own for the long buckets); it is where the radix sort changes its form too.
+#define CAFE_JOB_MOST 131072     // most lookups of a job's call
+// (the timeline's steps take one position or op per thread there: a chain of dependent loads each, so four or eight in a row
+// per thread, as in the launches of their own, took 6 to 19 us a step)
+#define CAFE_JOB_RESIDENT 3      // blocks per SM (the list replay takes 168 registers)
+
+enum { CAFE_JOB_DONE = 0, CAFE_JOB_ROUND_CAP = 1, CAFE_JOB_ERROR = 2, CAFE_JOB_EMPTY = 3 };
+struct CafeJobRun {
+    CafeHot hot1, hot2;
+    int32_t *beg1, *beg2;
+    uint8_t* marks[2];
+    CafeRoundResult* res;        // [2], taking turns
+    uint32_t* ring;
+    double refit_above;          // a re-fit is due at the first boundary with more crossings than this
+    int32_t real_n, adjust, round_cap, units;   // units: groups of 32 buckets a warp scans in a later round
+    CafeJobOutcome* out;         // in host memory
+};
+union CafeJobShared {
+    struct {
+        float c[4][CAFE_STAGE_MAIN];
+        float d[4][CAFE_STAGE_MAIN];
+        int p[4][CAFE_STAGE_MAIN];
+        uint32_t x[4][CAFE_STAGE_MAIN], kf[4][CAFE_STAGE_MAIN];
+    } main;
+    CafeLruStage lru[4];
+    struct { int warp[CAFE_JOB_THREADS / 32]; int cross; CafeFn fn[CAFE_JOB_THREADS / 32]; CafeFn before; } tl;
+    __device__ CafeJobShared() {}
+};
+
+// The buckets of one pass: every listed bucket and every group of buckets is a unit, and units go to the warps of the grid in
+// order, listed ones (the long ones) first.  wanted(k): does bucket k replay in this round.
+template <typename WANTED, typename LISTED, typename SHORT>
+__device__ __forceinline__ void cafe_job_units(const CafeHot& H, const int nb, const int groups, const bool all, int* s_q,
+                                               const WANTED& wanted, const LISTED& listed, const SHORT& replay) {
+    const int lane = threadIdx.x & 31;
+    const int warp = blockIdx.x * (CAFE_JOB_THREADS / 32) + (threadIdx.x >> 5), warps = gridDim.x * (CAFE_JOB_THREADS / 32);
+    const int n_hot = min(H.count[0], CAFE_HOT_CAP), n_list = n_hot + min(H.count[1], H.cap2);
+    for (int u = warp; u < n_list; u += warps) listed(lane == 0 ? H.list[u < n_hot ? u : CAFE_HOT_CAP + (u - n_hot)] : nb);
+    // (warps from the far end take groups first: those at the front are busy with the list)
+    const int per = all ? 1 : groups, chunks = (nb + 32 * per - 1) / (32 * per);
+    for (int u = warps - 1 - warp; u < chunks; u += warps) {
+        const int lo = u * per * 32;
+        int nq = 0;
+        for (int it = 0; it < per; ++it) {
+            const int k = lo + it * 32 + lane;
+            const bool a = k < nb && (all || (wanted(k) && !H.flag[k]));
+            const unsigned m = __ballot_sync(CAFE_FULL, a);
+            if (a) s_q[nq + __popc(m & ((1u << lane) - 1u))] = k;
+            nq += __popc(m);
+        }
+        __syncwarp();
+        for (int q0 = 0; q0 < nq; q0 += 32) replay(q0 + lane < nq ? s_q[q0 + lane] : nb);
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(CAFE_JOB_THREADS, CAFE_JOB_RESIDENT)
+k_whole_job(const __grid_constant__ CafeJob J0, const __grid_constant__ CafeJobRun P) {
+    __shared__ CafeJob J;
+    __shared__ __align__(16) CafeJobShared S;
+    __shared__ int s_q[4][CAFE_SCAN_MAIN];
+    __shared__ int s_next, s_from, s_to;
+    constexpr int T = CAFE_JOB_THREADS;
+    namespace cg = cooperative_groups;
+    cg::grid_group grid = cg::this_grid();
+    const size_t tid = (size_t)blockIdx.x * T + threadIdx.x, nth = (size_t)gridDim.x * T;
+    const int wib = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < (int)(sizeof(CafeJob) / 4); i += T) reinterpret_cast<uint32_t*>(&J)[i] = reinterpret_cast<const uint32_t*>(&J0)[i];
+    const int n1 = J0.n1, n2 = J0.n2, begin = J0.begin;
+    {   // the job's window: no results, no events, no visitors yet
+        const size_t span = (size_t)(J0.limit - begin);
+        cafe_fill(J0.ins_res + begin, 0, 4 * span, tid, nth);
+        cafe_fill(J0.mflag + begin, 0, span, tid, nth);
+        cafe_fill(J0.ev + begin, 0, sizeof(CafeEvent) * span, tid, nth);
+        cafe_fill(J0.mark2, 0, (size_t)n2, tid, nth);
+        cafe_fill(P.res, 0, sizeof(CafeRoundResult), tid, nth);
+        if (J0.post_row) cafe_fill(J0.post_row + begin, 0, 4 * span, tid, nth);
+    }
+    grid.sync();
+    int par = 0, rounds = 0, truncated = 0, state = CAFE_JOB_DONE;
+    for (;;) {
+        if (threadIdx.x == 0 && !J.final_pass) {
+            J.res = P.res + (rounds & 1);
+            J.mark_in1 = P.marks[par]; J.mark_out1 = P.marks[par ^ 1];
+            J.first_round = J.all_active = rounds == 0 ? 1 : 0;
+        }
+        __syncthreads();
+        cafe_job_units(P.hot1, n1, P.units, J.all_active != 0, s_q[wib],
+                       [&](int k) { bool cond; return CafeMainReplay::wanted(J, k, &cond); },
+                       [&](int k) { cafe_main_body<0>(J, P.hot1, k, S.main.c, S.main.p, S.main.x, S.main.kf, S.main.d); },
+                       [&](int k) { cafe_main_body<1>(J, P.hot1, k, S.main.c, S.main.p, S.main.x, S.main.kf); });
+        if (J.final_pass) break;
+        grid.sync();
+        cafe_job_units(P.hot2, n2, 1, J.all_active != 0, s_q[wib],
+                       [&](int k) { bool cond; return CafeLruReplay::wanted(J, k, &cond); },
+                       [&](int k) { cafe_lru_body<0>(J, P.hot2, k, &S.lru[wib]); },
+                       [&](int k) { cafe_lru_body<1>(J, P.hot2, k, nullptr); });
+        grid.sync();
+        // what the next round (or the final pass) routes events into, its result, and this round's ops and misses
+        const int ntl = (J.limit - begin + T - 1) / T;
+        cafe_fill(J0.head, 0xff, 4 * (size_t)n1, tid, nth);
+        cafe_fill(J0.mark_own, 0, (size_t)n1, tid, nth);
+        cafe_fill(J0.mark2, 0, (size_t)n2, tid, nth);
+        cafe_fill(P.res + ((rounds + 1) & 1), 0, sizeof(CafeRoundResult), tid, nth);
+        for (int blk = blockIdx.x; blk < ntl; blk += gridDim.x) cafe_tl_count_block<T, 1>(J, blk, ntl, S.tl.warp, &S.tl.cross);
+        grid.sync();
+        for (int blk = blockIdx.x; blk < ntl; blk += gridDim.x) cafe_tl_emit_block<T, 1>(J, blk, ntl, S.tl.warp);
+        for (int64_t p = begin + (int64_t)tid; p < J.limit; p += nth) cafe_route_position(J, (int)p);
+        grid.sync();
+        const int32_t n_ops = J.tl_head[0];
+        if (n_ops > T) {
+            cafe_tl_aggregate_blocks<T, 1>(J, S.tl.fn);
+            grid.sync();
+        }
+        if (n_ops > 0) {
+            cafe_tl_finish_blocks<T, 1>(J, S.tl.fn, &S.tl.before);
+            grid.sync();
+        }
+        // the decision, by every block for itself
+        ++rounds;
+        par ^= 1;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const CafeRoundResult* R = J.res;
+            s_next = R->error ? -1 : (R->changed ? 1 : 0);   // -1 stop, -2 nothing left, 0 converged, 1 another round, 2 shortened
+            s_from = s_to = 0;
+            if (P.adjust && !R->error) {
+                int rn = P.real_n;
+                for (int b = 1; b < J.nseg; ++b) {
+                    rn += R->seg_real_delta[b - 1];
+                    if ((double)rn > P.refit_above) {
+                        s_from = J.seg_off[b]; s_to = J.limit;
+                        J.limit = J.seg_off[b]; J.nseg = b;
+                        s_next = J.limit == begin ? -2 : 2;
+                        break;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        const int next = s_next;
+        if (next == -1) { state = CAFE_JOB_ERROR; break; }
+        if (next == -2) { truncated = 1; state = CAFE_JOB_EMPTY; break; }
+        if (next != 0 && rounds >= P.round_cap) { truncated |= next == 2; state = CAFE_JOB_ROUND_CAP; break; }
+        if (next == 2) {
+            // what the dropped lookups touched replays, and events are routed without theirs
+            truncated = 1;
+            for (int64_t p = s_from + (int64_t)tid; p < s_to; p += nth) cafe_mark_cut_position(J, (int)p, P.marks[par]);
+            cafe_fill(J0.head, 0xff, 4 * (size_t)n1, tid, nth);
+            cafe_fill(J0.mark_own, 0, (size_t)n1, tid, nth);
+            grid.sync();
+            for (int64_t p = begin + (int64_t)tid; p < J.limit; p += nth) cafe_route_position(J, (int)p);
+            grid.sync();
+        }
+        if (next == 0) {
+            if (threadIdx.x == 0) { J.first_round = J.all_active = 0; J.final_pass = 1; }
+            if (!J0.post_row) break;
+        }
+    }
+    __syncthreads();
+    if (blockIdx.x == 0) {
+        const uint32_t* r = reinterpret_cast<const uint32_t*>(J.res);
+        for (int i = threadIdx.x; i < (int)(sizeof(CafeRoundResult) / 4); i += T) reinterpret_cast<uint32_t*>(&P.out->r)[i] = r[i];
+        if (threadIdx.x == 0) { P.out->state = state; P.out->rounds = rounds; P.out->nseg = J.nseg; P.out->limit = J.limit; P.out->truncated = truncated; }
+    }
+    if (state != CAFE_JOB_DONE) return;
+    const int ntl = (J.limit - begin + T - 1) / T;
+    for (int blk = blockIdx.x; blk < ntl; blk += gridDim.x) cafe_miss_prefix_block<T, 1>(J, blk, S.tl.warp);
+    for (int64_t p = begin + (int64_t)tid; p < J.limit; p += nth) cafe_finalize_position(J, (int)p);
+    grid.sync();
+    for (int64_t k = tid; k < n2; k += nth) {
+        cafe_lru_tconvert(J, (int)k);
+        P.beg2[k] = cafe_advance_cursor(J.ord2, P.beg2[k], J.start2[k + 1], J.limit);
+    }
+    for (int64_t k = tid; k < n1; k += nth) P.beg1[k] = cafe_advance_cursor(J.ord1, P.beg1[k], J.start1[k + 1], J.limit);
+    const int32_t n_push = J.res->n_push, n_pop_ok = J.res->n_pop_ok;
+    for (int64_t j = tid; j < n_push; j += nth) cafe_commit_push(P.ring, J.ring_mask, J.q_head, J.q_size, n_pop_ok, J.pushbuf, (int)j);
 }
 __global__ void k_commit_queue(uint32_t* ring, uint32_t mask, uint32_t q_head, int32_t q_size, int32_t n_pop_ok,
                                const uint32_t* __restrict__ pushbuf, int n_push) {
@@ -1576,6 +1804,9 @@ struct CudaBackend {
     int hot_nb[2] = {0, 0};
     int cap = 0;
     void* pinned = nullptr;   // staging for small device-to-host reads
+    CafeRoundResult* job_res = nullptr;   // [2] round results of the whole-job launch
+    CafeJobOutcome* job_out = nullptr;    // what it reports, in host memory
+    int job_blocks = 0;                   // blocks of it that are resident at once (0: no cooperative launches here)
 
     ~CudaBackend() {
         if (cub_tmp) cudaFree(cub_tmp);
@@ -1597,6 +1828,8 @@ struct CudaBackend {
         for (int i = 0; i < 2; ++i) { if (hot_list[i]) cudaFree(hot_list[i]); if (hot_flag[i]) cudaFree(hot_flag[i]); }
         if (hot_count[0]) cudaFree(hot_count[0]);
         if (pinned) cudaFreeHost(pinned);
+        if (job_res) cudaFree(job_res);
+        if (job_out) cudaFreeHost(job_out);
     }
     void check(cudaError_t e) { if (e != cudaSuccess && err == cudaSuccess) err = e; }
     void check_launch() { check(cudaGetLastError()); }
@@ -1666,6 +1899,16 @@ struct CudaBackend {
         check(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
         check(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
         check(cudaMallocHost(&pinned, 4096));
+        check(cudaMalloc(&job_res, 2 * sizeof(CafeRoundResult)));
+        check(cudaMallocHost(&job_out, sizeof(CafeJobOutcome)));
+        {
+            int dev = 0, coop = 0, sms = 0, per = 0;
+            check(cudaGetDevice(&dev));
+            check(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+            check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_whole_job, CAFE_JOB_THREADS, 0));
+            job_blocks = coop ? sms * per : 0;
+        }
         hot_nb[0] = n1; hot_nb[1] = n2;
         check(cudaMalloc(&miss.pre, 4 * ((size_t)cap + 1)));
         check(cudaMalloc(&miss.list, 4 * (size_t)cap));
@@ -1796,6 +2039,30 @@ struct CudaBackend {
         }
         pass_join();
         check_launch();
+    }
+    // A job the resident grid can carry, rounds and commit in one launch; false: the engine takes the steps itself.  Lookups
+    // that outnumber the LRU buckets 256 times go by the compacted lists, which only the launches have.
+    bool run_job(const CafeJob& J0, uint8_t* const marks[2], uint32_t* ring, double refit_above, int real_n, bool adjust,
+                 int round_cap, CafeJobOutcome* out) {
+        if (job_blocks < 1 || cafe_prof_serialise() || J0.M > CAFE_JOB_MOST || (int64_t)J0.M >= 256 * (int64_t)J0.n2) return false;
+        CafeJob J = J0;
+        J.memo1 = memo1;
+        CafeJobRun P;
+        P.hot1 = hot(0); P.hot2 = hot(1);
+        P.beg1 = const_cast<int32_t*>(J.beg1); P.beg2 = const_cast<int32_t*>(J.beg2);
+        P.marks[0] = marks[0]; P.marks[1] = marks[1];
+        P.res = job_res; P.ring = ring; P.out = job_out;
+        P.refit_above = refit_above; P.real_n = real_n; P.adjust = adjust ? 1 : 0; P.round_cap = round_cap;
+        // a warp per 32 main buckets and some for the long ones; more blocks only make the barriers longer
+        const int blocks = std::min(job_blocks, cafe_blocks((int64_t)J.n1 / 32 + 128, CAFE_JOB_THREADS / 32));
+        P.units = std::min(CAFE_SCAN_MAIN / 32, std::max(1, cafe_blocks(J.n1, 32 * blocks * (CAFE_JOB_THREADS / 32))));
+        void* args[] = {&J, &P};
+        sort_join(0);
+        CAFE_PROF(CAFE_P_MAIN, stream);
+        check(cudaLaunchCooperativeKernel((const void*)k_whole_job, dim3((unsigned)blocks), dim3(CAFE_JOB_THREADS), args, 0, stream));
+        check(cudaStreamSynchronize(stream));
+        if (ok()) *out = *job_out;
+        return true;
     }
     void mark_cut(const CafeJob& J, int from, int to, uint8_t* mark_next1) {
         if (to <= from) return;

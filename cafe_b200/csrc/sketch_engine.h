@@ -16,6 +16,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "sketch_core.cuh"
@@ -24,6 +25,15 @@ struct CafeSketchStats {
     int64_t calls, lookups, rounds, jobs, truncated_jobs, resets, resets_refused, flips;
     int64_t seq_fallbacks, main_hits, lru_visits, events, max_rounds;
 };
+
+// What a backend that runs whole jobs by itself (rounds, decisions, commit) reports about one.
+struct CafeJobOutcome {
+    CafeRoundResult r;   // of the last round
+    int32_t state;       // 0 committed, 1 round cap reached, 2 inconsistency, 3 nothing left after a shortening
+    int32_t rounds, nseg, limit, truncated;   // truncated: the job was shortened at a re-fit
+};
+template <class BE, class = void> struct CafeRunsJobs : std::false_type {};
+template <class BE> struct CafeRunsJobs<BE, std::void_t<decltype(&BE::run_job)>> : std::true_type {};
 
 template <class BE>
 class SketchEngine {
@@ -105,8 +115,8 @@ public:
         tl_grp = (int32_t*)be.alloc(4 * (M / CAFE_TL_GROUP + 2));
         tl_head = (int32_t*)be.alloc(4 * 4);
         pushbuf = (uint32_t*)be.alloc(4 * M);
-        tl_blk = (int32_t*)be.alloc(4 * 2 * (M / CAFE_TL_BLOCK + 2));
-        tl_agg = (CafeFn*)be.alloc(sizeof(CafeFn) * (2 * M / CAFE_TL_BLOCK + 2));
+        tl_blk = (int32_t*)be.alloc(4 * 2 * (M / CAFE_TL_SMALL + 2));
+        tl_agg = (CafeFn*)be.alloc(sizeof(CafeFn) * (2 * M / CAFE_TL_SMALL + 2));
         nmiss = (int32_t*)be.alloc(4 * M);
         ins_res = (int32_t*)be.alloc(4 * M);
         seq_dev = (CafeSeqState*)be.alloc(sizeof(CafeSeqState));
@@ -415,6 +425,22 @@ private:
         ++stats.jobs;
         if (++job_serial <= 0) job_serial = 1;
         J.serial = job_serial;
+        if constexpr (CafeRunsJobs<BE>::value) {
+            CafeJobOutcome O;
+            uint8_t* const marks[2] = {mark_w1[mark_par], mark_w1[mark_par ^ 1]};
+            if (be.run_job(J, marks, ring, lim * 1.2, real_n, adjust != 0, round_cap, &O)) {
+                if (!be.ok()) return last_status = CAFE_ERR_CUDA;
+                if (O.rounds & 1) mark_par ^= 1;
+                stats.rounds += O.rounds;
+                stats.truncated_jobs += O.truncated;
+                if (O.state == 1) return sequential_fallback(J, done);
+                if (O.state == 2) return last_status = CAFE_ERR_CAPACITY;
+                if (O.state == 3) { *done = O.nseg; return CAFE_OK; }
+                cursors_advanced = true;
+                J.limit = O.limit;
+                return account(J, O.r, O.nseg, O.rounds, done);
+            }
+        }
         {
             const size_t span = (size_t)(J.limit - J.begin);
             be.fills(ins_res + J.begin, 0, 4 * span, mflag + J.begin, 0, span,
@@ -428,15 +454,7 @@ private:
         int dropped_from = 0, dropped_to = 0;   // positions a shortening has just dropped from the job
         bool first = true;
         for (;;) {
-            if (rounds >= round_cap) {
-                // state untouched so far (rounds only write the other image): sequential fallback
-                ++stats.seq_fallbacks;
-                last_status = CAFE_ERR_NOCONVERGE;
-                *done = 1;
-                const int b0 = J.begin, n0 = J.seg_off[1] - J.begin;
-                int rc = run_sequential(gid + b0, imp ? imp + b0 : nullptr, n0, mask + b0, post_row ? post_row + b0 : nullptr);
-                return rc == CAFE_OK ? CAFE_OK : rc;
-            }
+            if (rounds >= round_cap) return sequential_fallback(J, done);
             J.first_round = first ? 1 : 0;
             J.mark_in1 = mark_w1[mark_par]; J.mark_out1 = mark_w1[mark_par ^ 1];
             mark_par ^= 1;   // what this round marks is what the next one reads
@@ -500,6 +518,19 @@ private:
         be.finalize(J);   // per-lookup results, LRU clock values, cursors of the sorted order
         cursors_advanced = true;
         if (R.n_push > 0) be.commit_queue(ring, ring_mask, q_head, q_size, R.n_pop_ok, pushbuf, R.n_push);
+        return account(J, R, nseg, rounds, done);
+    }
+
+    // the job's first call by the sequential kernel: rounds only write the other image, so the state is untouched
+    int sequential_fallback(const CafeJob& J, int* done) {
+        ++stats.seq_fallbacks;
+        last_status = CAFE_ERR_NOCONVERGE;
+        *done = 1;
+        const int b0 = J.begin, n0 = J.seg_off[1] - J.begin;
+        return run_sequential(J.gid + b0, J.imp ? J.imp + b0 : nullptr, n0, J.mask + b0, J.post_row ? J.post_row + b0 : nullptr);
+    }
+    // the host's scalars after a job of nseg segments has been committed
+    int account(const CafeJob& J, const CafeRoundResult& R, int nseg, int rounds, int* done) {
         cur ^= 1;
         q_head += (uint32_t)R.n_pop_ok;
         q_size += R.n_push - R.n_pop_ok;

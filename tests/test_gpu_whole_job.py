@@ -1,0 +1,56 @@
+"""Jobs that run in one launch (rounds, shortenings at re-fits, final pass, commit) against the same jobs taken step by step, a
+launch each (the form that per-kernel timing uses): the same masks, post-insert rows and states, over calls of one lookup
+up to the largest and one more, tables of one block and of many, several calls per job with re-fits falling due inside,
+decays, unit counts, empty calls, a round cap of one."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(step_by_step, lim, thr, alpha, calls, n, dom, fuse, unit, cap, seed):
+    import torch
+    from cafe_b200 import HotSketch, profile
+    rng = np.random.default_rng(seed)
+    sk = HotSketch(lim, thr, 1, alpha, max_lookups=n * fuse)
+    if cap:
+        sk.tune(round_cap=cap)
+    out = []
+    profile.enable(step_by_step)
+    try:
+        for c in range(calls):
+            sizes = [n] * fuse if fuse < 4 else [0 if f == c % fuse else 1 + (f * 37 + c * 11) % n for f in range(fuse)]
+            off = np.concatenate([[0], np.cumsum(sizes)])
+            m = int(off[-1])
+            ids = np.minimum((dom * rng.random(m) ** 3).astype(np.int64) + 1, dom).astype(np.int32)
+            imp = None if unit else torch.from_numpy((rng.random(m) * 2).astype(np.float32)).cuda()
+            mask, post = sk.insert(torch.from_numpy(ids).cuda(), imp, off.tolist())
+            out.append((mask.cpu().numpy(), np.where(mask.cpu().numpy() == 1, post.cpu().numpy(), 0), sk.last_status))
+    finally:
+        profile.enable(False)
+        profile.read()
+    return out, sk.state(), sk.stats()
+
+
+@pytest.mark.parametrize("lim,thr,alpha,calls,n,dom,fuse,unit,cap", [
+    (40, 1, 1.0000005, 6, 1, 60, 1, False, 0),
+    (40, 1, 1.3, 60, 96, 200, 1, False, 0),
+    (300, 1, 1.2, 40, 33, 3000, 13, False, 0),
+    (300, 2, 1.0000005, 12, 129, 900, 7, True, 0),
+    (2000, 1, 1.0000005, 10, 1024, 50_000, 26, False, 0),
+    (20_000, 1, 1.0000005, 8, 4096, 5_000_000, 26, False, 0),
+    (20_000, 3, 1.0000005, 4, 131_072, 200_000, 1, False, 0),
+    (20_000, 1, 1.0000005, 3, 131_073, 200_000, 1, False, 0),
+    (400_000, 1, 1.0000005, 4, 5000, 3_000_000, 20, False, 0),
+    (500, 1, 1.0000005, 6, 700, 2000, 3, False, 1),
+])
+def test_one_launch_equals_step_by_step(lim, thr, alpha, calls, n, dom, fuse, unit, cap):
+    from oracle.hotsketch import states_equal
+    a = _run(True, lim, thr, alpha, calls, n, dom, fuse, unit, cap, n + lim)
+    b = _run(False, lim, thr, alpha, calls, n, dom, fuse, unit, cap, n + lim)
+    for c, (u, v) in enumerate(zip(a[0], b[0])):
+        assert u[2] == v[2], c
+        assert np.array_equal(u[0], v[0]) and np.array_equal(u[1], v[1]), c
+    assert states_equal(a[1], b[1]) == []
+    keys = ("calls", "lookups", "resets", "flips", "seq_fallbacks", "main_hits", "lru_visits")   # (rounds may differ: passes race with withdrawals)
+    assert {k: a[2][k] for k in keys} == {k: b[2][k] for k in keys}
