@@ -10,6 +10,8 @@ struct CafeSortDesc;   // radix_sort.cuh
 
 #define CAFE_MAX_DIM 128      // widest embedding row the scatter workspace is sized for
 #define CAFE_CHUNK 32         // sorted lookups reduced by one thread group in the scatter
+#define CAFE_CHUNK_SMALL 8            // ... in calls of
+#define CAFE_CHUNK_SMALL_MOST 131072  // at most so many lookups
 
 struct CafeSketchView {
     const CafeMainBucket* main;
@@ -26,7 +28,7 @@ struct CafeEmbedWorkspace {
     int32_t* post_row = nullptr; // [cap] hot row after the lookup's own call
     uint32_t* key = nullptr;                 // [cap] unified row key of every lookup
     uint2* rows = nullptr;                   // [cap] (row key, position) sorted by row
-    float* partial = nullptr;    // [2 * ceil(cap/CAFE_CHUNK) * CAFE_MAX_DIM] partial row sums of chunk-spanning rows
+    float* partial = nullptr;    // [2 * chunks * CAFE_MAX_DIM] partial row sums of chunk-spanning rows
     int32_t* row_winner = nullptr;   // [hotn] migration: highest position that claims a hot row in this call (-1 between calls)
     uint2* rows_tmp = nullptr;       // [cap] pairs between two passes of the row sort
     const uint32_t* keys_of = nullptr;   // `key` was left by cafe_embed_resolve for the lookups whose global ids are in this array

@@ -299,17 +299,17 @@ __device__ __forceinline__ void sgd_apply(float* w, float4 g, float lr) {
 
 #define NOKEY 0xffffffffu
 
-template <int G>
+template <int G, int CH>
 __global__ void __launch_bounds__(256, 4)
 k_scatter_chunks(const __grid_constant__ CafeFields F, const float* __restrict__ grad, int64_t field_stride,
                  int64_t sample_stride, const uint2* __restrict__ rows, int M, float lr, float* __restrict__ partial) {
-    constexpr int PER = CAFE_CHUNK / G;   // sorted entries held per lane
+    constexpr int PER = (CH + G - 1) / G;   // sorted entries held per lane
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t chunk = t / G;
     const int gl = (int)(t % G);          // lane within the group
     const int c = gl * 4;
-    const int64_t base = chunk * CAFE_CHUNK;
-    const int cnt = (int)max((int64_t)0, min((int64_t)CAFE_CHUNK, (int64_t)M - base));
+    const int64_t base = chunk * CH;
+    const int cnt = (int)max((int64_t)0, min((int64_t)CH, (int64_t)M - base));
     uint32_t k[PER];
     int32_t q[PER];
 #pragma unroll
@@ -320,16 +320,16 @@ k_scatter_chunks(const __grid_constant__ CafeFields F, const float* __restrict__
         q[i] = (int32_t)e.y;
     }
     const uint32_t key_prev = (cnt > 0 && base > 0) ? rows[base - 1].x : NOKEY;
-    const uint32_t key_next = (cnt > 0 && base + CAFE_CHUNK < M) ? rows[base + CAFE_CHUNK].x : NOKEY;
+    const uint32_t key_next = (cnt > 0 && base + CH < M) ? rows[base + CH].x : NOKEY;
 
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t cur = NOKEY;
     int cur_pos = 0;
     bool first_seg = true;
     const int B = F.B;
-    constexpr int U = 8;
+    constexpr int U = CH < 8 ? CH : 8;
 #pragma unroll
-    for (int j0 = 0; j0 < CAFE_CHUNK; j0 += U) {
+    for (int j0 = 0; j0 < CH; j0 += U) {
         float4 v[U];
         uint32_t kk[U];
         int32_t qq[U];
@@ -371,39 +371,85 @@ k_scatter_chunks(const __grid_constant__ CafeFields F, const float* __restrict__
     }
 }
 
-// One group per chunk; the chunk in which a spanning row STARTS adds up that row's partial sums.
-template <int G>
-__global__ void __launch_bounds__(256)
-k_scatter_fixup(const __grid_constant__ CafeFields F, const uint2* __restrict__ rows, int M, float lr, const float* __restrict__ partial) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t chunk = t / G;
-    const int c = (int)(t % G) * 4;
-    const int64_t base = chunk * CAFE_CHUNK;
-    if (base + CAFE_CHUNK >= M) return;   // the last chunk cannot continue to the right
-    const uint2 last = rows[base + CAFE_CHUNK - 1];
-    const uint32_t key = last.x;
-    if (key != rows[base + CAFE_CHUNK].x) return;            // its last row ends with the chunk
-    const bool single = rows[base].x == key;
-    if (single && base > 0 && rows[base - 1].x == key) return;   // the row started in an earlier chunk
-    // end of the row's range in the sorted keys
-    int64_t lo = base + CAFE_CHUNK, hi = M;   // first index with key' > key lies in (lo, hi]
-    while (lo < hi) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (rows[mid].x <= key) lo = mid + 1; else hi = mid;
-    }
-    const int64_t last_chunk = (lo - 1) / CAFE_CHUNK;
-    float4 acc = *reinterpret_cast<const float4*>(partial + (size_t)(chunk * 2 + (single ? 0 : 1)) * CAFE_MAX_DIM + c);
+// One group per chunk; the chunk in which a spanning row STARTS adds up that row's partial sums, in chunk order.  The rows at
+// the head of a skewed field span hundreds of chunks (33 000 lookups in one call: a thousand), which one group would add up
+// in a chain of loads that the whole launch waits for, so a row of more than CAFE_FIXUP_LONG chunks is shared out: every
+// group of the block adds up a stretch of it, and the group that found it adds the stretches in order: 37 us instead of 93
+// for 26 x 65536 lookups in a small sketch, 46 instead of 51 in a large one.
+#define CAFE_FIXUP_LONG 16
+// partial sums of the chunks [c0, c1) of a row, in order
+__device__ __forceinline__ float4 cafe_partial_sum(const float* __restrict__ partial, int64_t c0, int64_t c1, int c) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     constexpr int U = 8;
-    for (int64_t c0 = chunk + 1; c0 <= last_chunk; c0 += U) {
+    for (; c0 < c1; c0 += U) {
         float4 v[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (c0 + u <= last_chunk) v[u] = *reinterpret_cast<const float4*>(partial + (size_t)((c0 + u) * 2) * CAFE_MAX_DIM + c);
+            if (c0 + u < c1) v[u] = *reinterpret_cast<const float4*>(partial + (size_t)((c0 + u) * 2) * CAFE_MAX_DIM + c);
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (c0 + u <= last_chunk) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
+            if (c0 + u < c1) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
     }
-    sgd_apply(row_ptr(F, key, (int)last.y) + c, acc, lr);
+    return acc;
+}
+template <int G, int CH>
+__global__ void __launch_bounds__(256)
+k_scatter_fixup(const __grid_constant__ CafeFields F, const uint2* __restrict__ rows, int M, float lr, const float* __restrict__ partial) {
+    constexpr int NG = 256 / G;
+    __shared__ float4 s_sum[256];
+    __shared__ int s_first[NG], s_count[NG];   // a long row's first continued chunk and how many follow
+    const int g = threadIdx.x / G, gl = threadIdx.x % G, c = gl * 4;
+    const int64_t chunk = (int64_t)blockIdx.x * NG + g;
+    const int64_t base = chunk * CH;
+    uint2 last = make_uint2(0u, 0u);
+    int more = 0;                 // chunks after this one that the row goes on into (0: nothing starts here)
+    bool single = false;
+    if (base + CH < M) {          // the last chunk cannot continue to the right
+        last = rows[base + CH - 1];
+        single = rows[base].x == last.x;
+        // its last row goes on to the right, and did not start in an earlier chunk
+        if (last.x == rows[base + CH].x && !(single && base > 0 && rows[base - 1].x == last.x)) {
+            // the row's end: strides that double until they overshoot, then between the last two
+            int64_t lo = base + CH, hi = lo + 1, stride = CH;   // rows[lo] is still the row's
+            for (;;) {
+                hi = lo + stride;
+                if (hi >= M) { hi = M; break; }
+                if (rows[hi].x != last.x) break;
+                lo = hi; stride *= 4;
+            }
+            while (hi - lo > 1) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (rows[mid].x == last.x) lo = mid; else hi = mid;
+            }
+            more = (int)(lo / CH - chunk);
+        }
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (more > 0) acc = *reinterpret_cast<const float4*>(partial + (size_t)(chunk * 2 + (single ? 0 : 1)) * CAFE_MAX_DIM + c);
+    if (more > 0 && more <= CAFE_FIXUP_LONG) {
+        const float4 v = cafe_partial_sum(partial, chunk + 1, chunk + 1 + more, c);
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        sgd_apply(row_ptr(F, last.x, (int)last.y) + c, acc, lr);
+    }
+    if (gl == 0) { s_first[g] = (int)(chunk + 1); s_count[g] = more > CAFE_FIXUP_LONG ? more : 0; }
+    if (!__syncthreads_or(more > CAFE_FIXUP_LONG)) return;
+    for (int r = 0; r < NG; ++r) {
+        const int n = s_count[r];
+        if (n == 0) continue;   // block-uniform
+        const int each = (n + NG - 1) / NG;
+        const int64_t from = (int64_t)s_first[r] + min(n, g * each), to = (int64_t)s_first[r] + min(n, (g + 1) * each);
+        s_sum[threadIdx.x] = cafe_partial_sum(partial, from, to, c);
+        __syncthreads();
+        if (g == r) {
+#pragma unroll 4
+            for (int q = 0; q < NG; ++q) {
+                const float4 v = s_sum[q * G + gl];
+                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            }
+            sgd_apply(row_ptr(F, last.x, (int)last.y) + c, acc, lr);
+        }
+        __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -594,7 +640,8 @@ __global__ void k_labels_to_float(const int32_t* __restrict__ label, int B, floa
 int cafe_embed_ws_init(CafeEmbedWorkspace* ws, int cap, int hotn) {
     ws->cap = cap;
     const size_t M = (size_t)cap;
-    const size_t chunks = (M + CAFE_CHUNK - 1) / CAFE_CHUNK;
+    const size_t small = M < CAFE_CHUNK_SMALL_MOST ? M : CAFE_CHUNK_SMALL_MOST;
+    const size_t chunks = (M + CAFE_CHUNK - 1) / CAFE_CHUNK + (small + CAFE_CHUNK_SMALL - 1) / CAFE_CHUNK_SMALL;
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t n) { if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1); };
     A((void**)&ws->norm, 4 * M); A((void**)&ws->imp, 4 * M); A((void**)&ws->totals, 4 * CAFE_MAX_SEGMENTS);
@@ -657,12 +704,12 @@ static int fill_fields(CafeFields* F, int nfields, int B, int D, int hotn, const
 
 static bool strides_ok(const float* p, int64_t fs, int64_t ss) { return aligned16(p) && fs % 4 == 0 && ss % 4 == 0; }
 
-#define DISPATCH_G(D, CALL)              \
+#define DISPATCH_G(D, ...)               \
     switch ((D) / 4) {                   \
-        case 4: { constexpr int G = 4; CALL; } break;   \
-        case 8: { constexpr int G = 8; CALL; } break;   \
-        case 16: { constexpr int G = 16; CALL; } break; \
-        default: { constexpr int G = 32; CALL; } break; \
+        case 4: { constexpr int G = 4; __VA_ARGS__; } break;   \
+        case 8: { constexpr int G = 8; __VA_ARGS__; } break;   \
+        case 16: { constexpr int G = 16; __VA_ARGS__; } break; \
+        default: { constexpr int G = 32; __VA_ARGS__; } break; \
     }
 
 // A forward has (re)written these two arrays: a head start or row keys left for arrays at the same addresses (of a
@@ -944,13 +991,20 @@ static int scatter_prepare(CafeEmbedWorkspace* ws, const CafeFields& F, const in
 
 static int scatter_apply(CafeEmbedWorkspace* ws, const CafeFields& F, const float* grad_dev, int64_t field_stride,
                          int64_t sample_stride, int total, int D, float lr, cudaStream_t st) {
-    const int64_t chunks = ((int64_t)total + CAFE_CHUNK - 1) / CAFE_CHUNK;
+    // Chunks of 32 lookups make the fewest partial sums; while they are too few to fill the GPU's warps the launch is bound
+    // by one group's walk over its chunk, and chunks of 8 shorten that: 26 x 128 lookups of D 16 take 5.2 us (19 in chunks of
+    // 32), 9 x 4096 of D 16 6.0 (23), 26 x 2048 of D 128 11 (22).  The line lies where 32-lookup chunks of the widest rows
+    // make a full wave of warps (4096 of them); there is room for the partial sums of short chunks up to it.
+    const bool small = total <= CAFE_CHUNK_SMALL_MOST;
+    const int64_t len = small ? CAFE_CHUNK_SMALL : CAFE_CHUNK, chunks = ((int64_t)total + len - 1) / len;
     { CAFE_PROF(CAFE_P_SCATTER, st);
-    DISPATCH_G(D, (k_scatter_chunks<G><<<(unsigned)((chunks * G + 255) / 256), 256, 0, st>>>(F, grad_dev, field_stride,
-                   sample_stride, ws->rows, total, lr, ws->partial))); }
+    DISPATCH_G(D, const unsigned blocks = (unsigned)((chunks * G + 255) / 256);
+        if (small) k_scatter_chunks<G, CAFE_CHUNK_SMALL><<<blocks, 256, 0, st>>>(F, grad_dev, field_stride, sample_stride, ws->rows, total, lr, ws->partial);
+        else k_scatter_chunks<G, CAFE_CHUNK><<<blocks, 256, 0, st>>>(F, grad_dev, field_stride, sample_stride, ws->rows, total, lr, ws->partial)); }
     { CAFE_PROF(CAFE_P_FIXUP, st);
-    DISPATCH_G(D, (k_scatter_fixup<G><<<(unsigned)((chunks * G + 255) / 256), 256, 0, st>>>(F, ws->rows, total,
-                   lr, ws->partial))); }
+    DISPATCH_G(D, const unsigned blocks = (unsigned)((chunks * G + 255) / 256);
+        if (small) k_scatter_fixup<G, CAFE_CHUNK_SMALL><<<blocks, 256, 0, st>>>(F, ws->rows, total, lr, ws->partial);
+        else k_scatter_fixup<G, CAFE_CHUNK><<<blocks, 256, 0, st>>>(F, ws->rows, total, lr, ws->partial)); }
     return fail_cuda("cafe_scatter_sgd");
 }
 
