@@ -30,7 +30,8 @@ import torch
 import torch.nn as nn
 from torch.autograd.profiler import record_function
 
-from . import sizing, synthetic
+from . import _lib, sizing, synthetic
+from .sketch import _stream
 from .sk_embedding_bag import SKEmbeddingGroup
 
 
@@ -225,14 +226,13 @@ class _FusedDotInteraction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, emb):
-        from . import _lib
         lib = _lib.load()
         x, emb = x.contiguous(), emb.contiguous()
         B, F, D = emb.shape
         nv = F + 1
         out = torch.empty(B, D + nv * (nv - 1) // 2, dtype=torch.float32, device=emb.device)
-        st = torch.cuda.current_stream(emb.device).cuda_stream
         with torch.cuda.device(emb.device):
+            st = _stream()
             _lib.check(lib.cafe_dot_interaction_forward(x.data_ptr(), emb.data_ptr(), D, F * D, B, F, D, 0, out.data_ptr(),
                                                         out.shape[1], st), "cafe_dot_interaction_forward")
         ctx.save_for_backward(x, emb)
@@ -240,14 +240,13 @@ class _FusedDotInteraction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_out):
-        from . import _lib
         lib = _lib.load()
         x, emb = ctx.saved_tensors
         B, F, D = emb.shape
         g = grad_out.contiguous()
         gx, ge = torch.empty_like(x), torch.empty_like(emb)
-        st = torch.cuda.current_stream(emb.device).cuda_stream
         with torch.cuda.device(emb.device):
+            st = _stream()
             _lib.check(lib.cafe_dot_interaction_backward(x.data_ptr(), emb.data_ptr(), D, F * D, B, F, D, 0, g.data_ptr(),
                                                          g.shape[1], gx.data_ptr(), ge.data_ptr(), D, F * D, st),
                        "cafe_dot_interaction_backward")

@@ -18,6 +18,7 @@ Differences from the reference that a caller can see:
 from __future__ import annotations
 
 import ctypes
+from array import array
 
 import numpy as np
 import torch
@@ -29,7 +30,8 @@ from .sketch import HotSketch, _stream
 
 
 def _ptr_array(tensors):
-    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+    ptrs = array("Q", [t.data_ptr() for t in tensors])   # (filling a ctypes array element by element takes 5 us for 26)
+    return (ctypes.c_void_p * len(ptrs)).from_buffer(ptrs)
 
 
 def _i64_array(vals):
@@ -59,10 +61,12 @@ class _FieldSet:
         self.hotn = int(weight_high.shape[0])
 
     def ptrs(self):
-        _check_table(self.weight_high.data, "weight_high")
+        # (asked of the Parameters themselves: `.data` makes a tensor object per table, which for 26 tables took 33 us of a
+        # step's two calls each, against 14)
+        _check_table(self.weight_high, "weight_high")
         for w in self.weight_hash:
-            _check_table(w.data, "weight_hash")
-        return _ptr_array([w.data for w in self.weight_hash]), self.weight_high.data.data_ptr()
+            _check_table(w, "weight_hash")
+        return _ptr_array(self.weight_hash), self.weight_high.data_ptr()
 
     def forward(self, ids: torch.Tensor, out: torch.Tensor, field_stride: int, sample_stride: int):
         """ids [nf*B] field-major on the device; returns (gid, row) saved for the backward."""
@@ -99,15 +103,15 @@ class _FieldSet:
         gid = torch.empty(ids.numel(), dtype=torch.int32, device=ids.device)
         row = torch.empty(ids.numel(), dtype=torch.int32, device=ids.device)
         wp, hp = self.ptrs()
+        gp, rp = gid.data_ptr(), row.data_ptr()
         with torch.cuda.device(ids.device):
+            st = _stream()
             _lib.check(lib.cafe_embed_resolve(sk.handle, ids.data_ptr(), int(ids.dtype == torch.int64), self.nf, B,
-                                              self.f_offset, self.hash_size, self.hotn, gid.data_ptr(), row.data_ptr(),
-                                              _stream()), "cafe_embed_resolve")
-            _lib.check(lib.cafe_embed_backward_begin(sk.handle, gid.data_ptr(), row.data_ptr(), self.nf, B, self.hash_size,
-                                                     wp, hp, self.hotn, self.dim, mode, _stream()), "cafe_embed_backward_begin")
-            _lib.check(lib.cafe_embed_gather(sk.handle, row.data_ptr(), self.nf, B, self.hash_size, wp, hp, self.hotn,
-                                             self.dim, out.data_ptr(), field_stride, sample_stride, _stream()),
-                       "cafe_embed_gather")
+                                              self.f_offset, self.hash_size, self.hotn, gp, rp, st), "cafe_embed_resolve")
+            _lib.check(lib.cafe_embed_backward_begin(sk.handle, gp, rp, self.nf, B, self.hash_size, wp, hp, self.hotn, self.dim,
+                                                     mode, st), "cafe_embed_backward_begin")
+            _lib.check(lib.cafe_embed_gather(sk.handle, rp, self.nf, B, self.hash_size, wp, hp, self.hotn, self.dim,
+                                             out.data_ptr(), field_stride, sample_stride, st), "cafe_embed_gather")
         return gid, row
 
     def importance(self, grad: torch.Tensor, field_stride: int, sample_stride: int, B: int) -> torch.Tensor:

@@ -20,7 +20,8 @@ _STATE_ARRAYS = ["main_val", "main_cnt", "main_dic", "main_flip", "lru_val", "lr
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream as a raw handle (torch's own accessor for launchers: no Stream object is made)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _np_ptr(a: np.ndarray, typ):
