@@ -31,6 +31,7 @@ struct CafeJobOutcome {
     CafeRoundResult r;   // of the last round
     int32_t state;       // 0 committed, 1 round cap reached, 2 inconsistency, 3 nothing left after a shortening
     int32_t rounds, nseg, limit, truncated;   // truncated: the job was shortened at a re-fit
+    int32_t ticket;      // number of the job the record belongs to
 };
 template <class BE, class = void> struct CafeRunsJobs : std::false_type {};
 template <class BE> struct CafeRunsJobs<BE, std::void_t<decltype(&BE::run_job)>> : std::true_type {};
