@@ -204,10 +204,9 @@ k_grad_norm(const float* __restrict__ grad, int64_t field_stride, int64_t sample
     }
 }
 
-// one block per field: fixed-order sum of the field's norms
-__global__ void __launch_bounds__(1024) k_field_sum(const float* __restrict__ norm, int B, float* __restrict__ totals) {
+// fixed-order sum of a field's norms by a block of 1024 threads
+__device__ __forceinline__ float cafe_field_sum(const float* __restrict__ x, int B) {
     __shared__ float sh[1024];
-    const float* x = norm + (size_t)blockIdx.x * B;
     float s = 0.f;
     for (int i = threadIdx.x; i < B; i += 1024) s += x[i];
     sh[threadIdx.x] = s;
@@ -216,16 +215,42 @@ __global__ void __launch_bounds__(1024) k_field_sum(const float* __restrict__ no
         if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) totals[blockIdx.x] = sh[0];
+    return sh[0];
+}
+// one block per field
+__global__ void __launch_bounds__(1024) k_field_sum(const float* __restrict__ norm, int B, float* __restrict__ totals) {
+    const float tot = cafe_field_sum(norm + (size_t)blockIdx.x * B, B);
+    if (threadIdx.x == 0) totals[blockIdx.x] = tot;
+}
+
+__device__ __forceinline__ float cafe_importance(float norm, float tot, int B) {
+    // a field whose whole gradient is zero would give 0/0 in the reference; counts stay unchanged here
+    return tot > 0.f ? __fdiv_rn(__fmul_rn(norm, (float)B), tot) : 0.f;
+}
+// both for one field per block, where a field is small enough that its block does not take longer than a second launch
+// (2.5 us, and as much again between launches)
+#define CAFE_FIELD_BLOCK_MOST 8192
+__global__ void __launch_bounds__(1024) k_field_importance(const float* __restrict__ norm, int B, float* __restrict__ totals, float* __restrict__ imp) {
+    const float tot = cafe_field_sum(norm + (size_t)blockIdx.x * B, B);
+    if (threadIdx.x == 0) totals[blockIdx.x] = tot;
+    for (int i = threadIdx.x; i < B; i += 1024) imp[(size_t)blockIdx.x * B + i] = cafe_importance(norm[(size_t)blockIdx.x * B + i], tot, B);
 }
 
 __global__ void k_importance(const float* __restrict__ norm, const float* __restrict__ totals, int B, int total,
                              float* __restrict__ imp) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= total) return;
-    const float tot = totals[p / B];
-    // a field whose whole gradient is zero would give 0/0 in the reference; counts stay unchanged here
-    imp[p] = tot > 0.f ? __fdiv_rn(__fmul_rn(norm[p], (float)B), tot) : 0.f;
+    imp[p] = cafe_importance(norm[p], totals[p / B], B);
+}
+// importance of nf fields from their norms
+static void field_importance(const float* norm, float* totals, int nf, int B, float* imp, cudaStream_t st) {
+    if (B <= CAFE_FIELD_BLOCK_MOST) {
+        CAFE_PROF(CAFE_P_IMPORTANCE, st);
+        k_field_importance<<<nf, 1024, 0, st>>>(norm, B, totals, imp);
+        return;
+    }
+    { CAFE_PROF(CAFE_P_FIELDSUM, st); k_field_sum<<<nf, 1024, 0, st>>>(norm, B, totals); }
+    { CAFE_PROF(CAFE_P_IMPORTANCE, st); k_importance<<<(unsigned)(((int64_t)nf * B + 255) / 256), 256, 0, st>>>(norm, totals, B, nf * B, imp); }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -872,8 +897,7 @@ int cafe_grad_importance(void* h, const float* grad_dev, int64_t field_stride, i
     { CAFE_PROF(CAFE_P_NORM, st);
     DISPATCH_G(D, (k_grad_norm<G><<<(unsigned)((((int64_t)total + 3) / 4 * G + 255) / 256), 256, 0, st>>>(grad_dev, field_stride,
                    sample_stride, B, total, ws->norm))); }
-    { CAFE_PROF(CAFE_P_FIELDSUM, st); k_field_sum<<<nfields, 1024, 0, st>>>(ws->norm, B, ws->totals); }
-    { CAFE_PROF(CAFE_P_IMPORTANCE, st); k_importance<<<(total + 255) / 256, 256, 0, st>>>(ws->norm, ws->totals, B, total, imp_out_dev); }
+    field_importance(ws->norm, ws->totals, nfields, B, imp_out_dev, st);
     return fail_cuda("cafe_grad_importance");
 }
 
@@ -938,8 +962,7 @@ int cafe_grad_importance_static(const float* grad_dev, int64_t field_stride, int
     cudaStream_t st = (cudaStream_t)stream;
     DISPATCH_G(D, (k_grad_norm<G><<<(unsigned)((((int64_t)total + 3) / 4 * G + 255) / 256), 256, 0, st>>>(grad_dev, field_stride,
                    sample_stride, B, total, norm)));
-    k_field_sum<<<nfields, 1024, 0, st>>>(norm, B, totals);
-    k_importance<<<(total + 255) / 256, 256, 0, st>>>(norm, totals, B, total, imp_out_dev);
+    field_importance(norm, totals, nfields, B, imp_out_dev, st);
     return fail_cuda("cafe_grad_importance_static");
 }
 
@@ -1078,9 +1101,7 @@ static int importance_range(CafeEmbedWorkspace* ws, const float* grad_dev, int64
     { CAFE_PROF(CAFE_P_NORM, st);
     DISPATCH_G(D, (k_grad_norm<G><<<(unsigned)((((int64_t)total + 3) / 4 * G + 255) / 256), 256, 0, st>>>(g, field_stride,
                    sample_stride, B, total, norm))); }
-    { CAFE_PROF(CAFE_P_FIELDSUM, st); k_field_sum<<<nf, 1024, 0, st>>>(norm, B, ws->totals + f0); }
-    { CAFE_PROF(CAFE_P_IMPORTANCE, st); k_importance<<<(total + 255) / 256, 256, 0, st>>>(norm, ws->totals + f0, B, total,
-                                                                                           imp_dev + (size_t)f0 * B); }
+    field_importance(norm, ws->totals + f0, nf, B, imp_dev + (size_t)f0 * B, st);
     return fail_cuda("cafe_grad_importance");
 }
 
@@ -1221,8 +1242,7 @@ int cafe_shard_pull_importance(void* h, const float* const* grad_rank, int nrank
     { CAFE_PROF(CAFE_P_NORM, st);
     DISPATCH_G(D, (k_pull_norm<G><<<(unsigned)((((int64_t)total + 3) / 4 * G + 255) / 256), 256, 0, st>>>(sb, field_stride,
                    sample_stride, B, total, local_grad_dev, ws->norm))); }
-    { CAFE_PROF(CAFE_P_FIELDSUM, st); k_field_sum<<<nfields, 1024, 0, st>>>(ws->norm, B, ws->totals); }
-    { CAFE_PROF(CAFE_P_IMPORTANCE, st); k_importance<<<(total + 255) / 256, 256, 0, st>>>(ws->norm, ws->totals, B, total, imp_out_dev); }
+    field_importance(ws->norm, ws->totals, nfields, B, imp_out_dev, st);
     return fail_cuda("cafe_shard_pull_importance");
 }
 
@@ -1353,9 +1373,7 @@ int cafe_embed_backward_norms(void* h, const float* grad_dev, int64_t field_stri
     if (rc != CAFE_OK) return rc;
     rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, insert_mode, st);
     if (rc != CAFE_OK) return rc;
-    { CAFE_PROF(CAFE_P_FIELDSUM, st); k_field_sum<<<nfields, 1024, 0, st>>>(norm_dev, B, ws->totals); }
-    { CAFE_PROF(CAFE_P_IMPORTANCE, st); k_importance<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(norm_dev, ws->totals, B,
-                                                                                                    (int)total, ws->imp); }
+    field_importance(norm_dev, ws->totals, nfields, B, ws->imp, st);
     int seg[CAFE_MAX_SEGMENTS + 1];
     for (int f = 0; f <= nfields; ++f) seg[f] = f * B;
     int status = cafe_internal_insert(h, gid_dev, ws->imp, seg, nfields, ws->mask, ws->post_row, insert_mode, true, st);

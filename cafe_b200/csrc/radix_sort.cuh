@@ -35,7 +35,7 @@
 #define CAFE_RS_MAX_SORTS 3
 #define CAFE_RS_CLUSTER_MAX 8           // portable cluster size
 // A cluster of eight blocks ranks 32 768 pairs at a time; up to four rounds of that cost less than the launches of the
-// other form.  The three sorts of a step with 26 x 128 lookups take 25 us in their one launch (the 23 launches of a
+// other form.  The three sorts of a step with 26 x 128 lookups take 17 us in their one launch (the 23 launches of a
 // launch per step, sort and bucket index took 84 us one after the other), with 26 x 2048 lookups 49 us (98 us); with
 // 26 x 65536, beside the row gather, 0.31 ms of kernel time in 7 launches (0.65 ms in 23).
 #define CAFE_RS_CLUSTER_PAIRS (4 * CAFE_RS_CLUSTER_MAX * CAFE_RS_TILE)
@@ -212,6 +212,84 @@ __device__ __forceinline__ void cafe_rs_starts(const CafeSortDesc& D, int warp, 
     }
 }
 
+// All passes of a sort whose blocks have at most a tile of pairs each: ranking the tile counts its digits as well, so there is
+// no histogram step, and the pairs are spread over all warps however few they are.
+// A sort of 2048 pairs by 18 638 buckets takes 12 us (21 with a histogram step and full tiles per warp), three sorts of 3328
+// pairs 17 us (25).  Half-filled blocks in a larger cluster beat full ones (3 x 8547 pairs: 17 us against 22).
+template <typename CLUSTER>
+__device__ __forceinline__ void cafe_rs_tiles(const CafeSortDesc& D, const CLUSTER& cluster, int nblk, int blk, CafeSortShared& S) {
+    const int bins = 1 << D.bits, d2 = (int)threadIdx.x * 2;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int64_t lo, hi;
+    cafe_rs_range(D, blk, &lo, &hi);
+    const int len = (int)(hi > lo ? hi - lo : 0), items = (len + CAFE_RS_THREADS - 1) / CAFE_RS_THREADS, first = w * 32 * items;
+    for (int pass = 0; pass < D.passes; ++pass) {
+        const int shift = pass * D.bits;
+        const uint2* from = cafe_rs_from(D, pass);
+        uint2* to = cafe_rs_to(D, pass);
+        uint2 e[CAFE_RS_ITEMS];
+        uint32_t dr[CAFE_RS_ITEMS];   // digit, and rank << 16
+#pragma unroll
+        for (int it = 0; it < CAFE_RS_ITEMS; ++it) {
+            const int i = first + it * 32 + lane;
+            e[it] = make_uint2(0u, 0u);
+            if (it < items && i < len) e[it] = pass == 0 ? make_uint2(D.in[lo + i], (uint32_t)(lo + i)) : from[lo + i];
+        }
+        {
+            uint4* z = reinterpret_cast<uint4*>(S.cnt[w]);
+            for (int q = lane; q < bins / 8; q += 32) z[q] = make_uint4(0u, 0u, 0u, 0u);
+            if (bins < 8 && lane < bins) S.cnt[w][lane] = 0;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < CAFE_RS_ITEMS; ++it) {
+            if (it >= items) break;   // block-uniform
+            const bool ok = first + it * 32 + lane < len;
+            const uint32_t d = (cafe_rs_key(D, e[it].x) >> shift) & (uint32_t)(bins - 1);
+            const unsigned peers = __match_any_sync(0xffffffffu, ok ? d : (uint32_t)(bins + lane));
+            const int ahead = __popc(peers & ((1u << lane) - 1u));
+            const uint32_t before = ok ? S.cnt[w][d] : 0u;
+            __syncwarp();
+            if (ok && ahead == 0) S.cnt[w][d] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+            dr[it] = d | ((before + ahead) << 16);
+        }
+        __syncthreads();   // (also: everyone has read its pairs)
+        uint32_t run = 0;
+        if (d2 < bins) {
+#pragma unroll
+            for (int q = 0; q < CAFE_RS_WARPS; ++q) {
+                uint32_t* c = reinterpret_cast<uint32_t*>(S.cnt[q]) + threadIdx.x;
+                const uint32_t t = *c;
+                *c = run;
+                run += t;
+            }
+        }
+        int loc[2] = {(int)(run & 0xffffu), (int)(run >> 16)}, own[2] = {0, 0};
+        if (nblk > 1) {
+            if (d2 < bins) { S.hist[d2] = loc[0]; S.hist[d2 + 1] = loc[1]; }
+            cluster.sync();
+            loc[0] = loc[1] = 0;
+            if (d2 < bins) {
+                for (int b = 0; b < nblk; ++b) {
+                    const int2 h = *reinterpret_cast<const int2*>(cluster.map_shared_rank(S.hist, b) + d2);
+                    loc[0] += h.x; loc[1] += h.y;
+                    if (b < blk) { own[0] += h.x; own[1] += h.y; }
+                }
+            }
+        }
+        cafe_rs_set_base(D, loc, own, S);   // (its barriers also publish the prefixes over the warps)
+#pragma unroll
+        for (int it = 0; it < CAFE_RS_ITEMS; ++it) {
+            if (it >= items) break;
+            const uint32_t d = dr[it] & 0xffffu;
+            if (first + it * 32 + lane < len) {
+                to[(int64_t)S.base[d] + S.cnt[w][d] + (dr[it] >> 16)] = e[it];
+            }
+        }
+        cluster.sync();
+    }
+}
 // a cluster per sort
 static __global__ void __launch_bounds__(CAFE_RS_THREADS) k_rs_cluster(const __grid_constant__ CafeSortBatch B) {
     __shared__ __align__(16) CafeSortShared S;
@@ -219,7 +297,9 @@ static __global__ void __launch_bounds__(CAFE_RS_THREADS) k_rs_cluster(const __g
     const int nblk = (int)cluster.num_blocks(), blk = (int)cluster.block_rank();
     const CafeSortDesc& D = B.d[blockIdx.x / nblk];
     const int bins = 1 << D.bits, d = (int)threadIdx.x * 2;
-    for (int pass = 0; pass < D.passes; ++pass) {
+    const bool tiles = ((((int64_t)D.n + nblk - 1) / nblk + 31) & ~(int64_t)31) <= CAFE_RS_TILE;
+    if (tiles) cafe_rs_tiles(D, cluster, nblk, blk, S);
+    for (int pass = 0; !tiles && pass < D.passes; ++pass) {
         cafe_rs_hist(D, pass, blk, S);
         cluster.sync();
         int loc[2] = {0, 0}, own[2] = {0, 0};

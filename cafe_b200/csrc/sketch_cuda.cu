@@ -124,9 +124,7 @@ struct CafeFindHot {
     uint8_t* flag;
     int32_t* beg;
 };
-__global__ void k_find_hot(const CafeFindHot A, const CafeFindHot B) {
-    const CafeFindHot& T = blockIdx.y == 0 ? A : B;
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void cafe_find_hot(const CafeFindHot& T, const int k) {
     if (k >= T.nb) return;
     const int s0 = T.start[k];
     const int len = T.start[k + 1] - s0;
@@ -144,6 +142,9 @@ __global__ void k_find_hot(const CafeFindHot A, const CafeFindHot B) {
         }
     }
     T.flag[k] = listed;
+}
+__global__ void k_find_hot(const CafeFindHot A, const CafeFindHot B) {
+    cafe_find_hot(blockIdx.y == 0 ? A : B, blockIdx.x * blockDim.x + threadIdx.x);
 }
 // next listed bucket for this warp (lane 0 owns it; -1 = none left); the cursor is zeroed with the round result
 __device__ __forceinline__ int cafe_next_listed(const CafeHot& H, int32_t* cursor, int nb) {
@@ -417,7 +418,7 @@ __device__ __forceinline__ void cafe_main_body(const CafeJob& J, const CafeHot& 
                     }                                                                                                     \
                 }
                 if (J.first_round && !J.final_pass && J.simp1) {
-                    const float* __restrict__ imp1 = J.simp1;
+                    const float* imp1 = J.simp1;   // (not __restrict__: the whole-job launch writes these counts itself)
                     while (good) {
                         CAFE_GROUP_STEP_FIRST(A, B, C)
                         if (!good) break;
@@ -1522,6 +1523,12 @@ struct CafeJobRun {
     int32_t real_n, adjust, round_cap, units;   // units: groups of 32 buckets a warp scans in a later round
     CafeJobOutcome* out;         // in host memory; complete once its ticket is this job's
     int32_t ticket;
+    // the first job of a call also does what lies between the sorts and the rounds: lists, flags and cursors of the buckets
+    // (into counters that the call before has cleared; it clears the others), counts in the two orders
+    int32_t first_of_call;
+    CafeFindHot find[2];
+    int32_t* other_count;        // [4]
+    float *simp1, *simp2;
 };
 union CafeJobShared {
     struct {
@@ -1593,6 +1600,16 @@ k_whole_job(const __grid_constant__ CafeJob J0, const __grid_constant__ CafeJobR
         cafe_fill(J0.mark2, 0, (size_t)n2, tid, nth);
         cafe_fill(P.res, 0, sizeof(CafeRoundResult), tid, nth);
         if (J0.post_row) cafe_fill(J0.post_row + begin, 0, 4 * span, tid, nth);
+    }
+    if (P.first_of_call) {
+        if (tid < 4) P.other_count[tid] = 0;
+        for (int64_t k = tid; k < n1; k += nth) cafe_find_hot(P.find[0], (int)k);
+        for (int64_t k = tid; k < n2; k += nth) cafe_find_hot(P.find[1], (int)k);
+        if (J0.simp1)
+            for (int64_t i = tid; i < J0.M; i += nth) {
+                P.simp1[i] = J0.imp[cafe_ord(J0.ord1, i)];
+                P.simp2[i] = J0.imp[cafe_ord(J0.ord2, i)];
+            }
     }
     grid.sync();
     int par = 0, rounds = 0, truncated = 0, state = CAFE_JOB_DONE;
@@ -1811,7 +1828,14 @@ struct CudaBackend {
     bool side_pending = false;
     int64_t* scan64 = nullptr;   // [4*(n1+n2)] prefix sums of the threshold re-fit
     int32_t* hot_list[2] = {nullptr, nullptr};   // listed long buckets of the main / LRU table
-    int32_t* hot_count[2] = {nullptr, nullptr};
+    int32_t* hot_counts = nullptr;               // [2 sets][2 tables][2 regions]; the sets take turns from call to call
+    int hot_set = 0;
+    bool find_pending = false;   // the lists of the last sort are left to the first job of the call
+    const float* gather_imp = nullptr;   // ... and so are these counts in its two orders
+    float *gather_simp1 = nullptr, *gather_simp2 = nullptr;
+    int32_t* count_of(int t) const { return hot_counts + 4 * hot_set + 2 * t; }
+    // jobs of the last sorted call go by the whole-job launch
+    bool carries(int64_t M, int n2) const { return job_blocks > 0 && !cafe_prof_serialise() && M <= CAFE_JOB_MOST && M < 256 * (int64_t)n2; }
     uint8_t* hot_flag[2] = {nullptr, nullptr};
     int hot_nb[2] = {0, 0};
     int cap = 0;
@@ -1839,7 +1863,7 @@ struct CudaBackend {
         if (miss.list) cudaFree(miss.list);
         if (miss.blk) cudaFree(miss.blk);
         for (int i = 0; i < 2; ++i) { if (hot_list[i]) cudaFree(hot_list[i]); if (hot_flag[i]) cudaFree(hot_flag[i]); }
-        if (hot_count[0]) cudaFree(hot_count[0]);
+        if (hot_counts) cudaFree(hot_counts);
         if (pinned) cudaFreeHost(pinned);
         if (job_res) cudaFree(job_res);
         if (job_out) cudaFreeHost(job_out);
@@ -1929,9 +1953,8 @@ struct CudaBackend {
         check(cudaMalloc(&miss.blk, 4 * ((size_t)cap / CAFE_TL_BLOCK + 2)));
         check(cudaMalloc(&memo1, sizeof(CafeCalmMemo) * (size_t)n1));
         check(cudaMemsetAsync(memo1, 0, sizeof(CafeCalmMemo) * (size_t)n1, stream));
-        check(cudaMalloc(&hot_count[0], 16));
-        hot_count[1] = hot_count[0] + 2;
-        check(cudaMemsetAsync(hot_count[0], 0, 16, stream));
+        check(cudaMalloc(&hot_counts, 32));
+        check(cudaMemsetAsync(hot_counts, 0, 32, stream));
         for (int i = 0; i < 2; ++i) {
             check(cudaMalloc(&hot_list[i], 4 * ((size_t)CAFE_HOT_CAP + (size_t)hot_nb[i])));
             check(cudaMalloc(&hot_flag[i], (size_t)hot_nb[i]));
@@ -1976,7 +1999,7 @@ struct CudaBackend {
         // load -- but never more than 64, beyond which one thread's serial replay is the tail whatever the average
         // (a sketch of a few thousand rows fed 65536-id calls has hundreds of lookups in EVERY bucket).
         CafeFindHot& F = find[t];
-        F.start = start; F.nb = nb; F.list = hot_list[t]; F.count = hot_count[t]; F.flag = hot_flag[t]; F.beg = beg;
+        F.start = start; F.nb = nb; F.list = hot_list[t]; F.flag = hot_flag[t]; F.beg = beg;
         F.hot_len = std::max(CAFE_HOT_LEN, std::min((int)(16.0 * M / nb), 4096));
         F.long_len = std::max(16, std::min((int)(4.0 * M / nb), 64));
         if (t == 1) return;
@@ -1991,10 +2014,9 @@ struct CudaBackend {
             CAFE_PROF(CAFE_P_LOOKUP_SORT, st);
             check(cafe_radix_sort(batch, st));
             batch.count = 0;
-            check(cudaMemsetAsync(hot_count[0], 0, 16, st));
-            const dim3 grid((unsigned)cafe_blocks(std::max(find[0].nb, find[1].nb)), 2);
-            k_find_hot<<<grid, CAFE_TPB, 0, st>>>(find[0], find[1]);
-            check_launch();
+            gather_imp = nullptr;
+            find_pending = carries(M, find[1].nb);
+            if (!find_pending) find_now(st);
         }
         if (aside) {
             check(cudaEventRecord(ev_join, side));
@@ -2002,7 +2024,17 @@ struct CudaBackend {
         }
     }
     CafeFindHot find[2];
+    void find_now(cudaStream_t st) {
+        find_pending = false;
+        hot_set ^= 1;
+        find[0].count = count_of(0); find[1].count = count_of(1);
+        check(cudaMemsetAsync(hot_counts, 0, 32, st));
+        const dim3 grid((unsigned)cafe_blocks(std::max(find[0].nb, find[1].nb)), 2);
+        k_find_hot<<<grid, CAFE_TPB, 0, st>>>(find[0], find[1]);
+        check_launch();
+    }
     void gather_counts(const float* imp, const int32_t* ord1, const int32_t* ord2, int M, float* simp1, float* simp2) {
+        if (find_pending) { gather_imp = imp; gather_simp1 = simp1; gather_simp2 = simp2; return; }
         CAFE_PROF(CAFE_P_LOOKUP_SORT, stream);
         k_gather_counts<<<cafe_blocks(M), CAFE_TPB, 0, stream>>>(imp, ord1, ord2, M, simp1, simp2);
         check_launch();
@@ -2033,7 +2065,7 @@ struct CudaBackend {
     }
     cudaEvent_t gate_event = nullptr;   // see SketchEngine::set_gate
     void wait_gate() { if (gate_event) check(cudaStreamWaitEvent(stream, gate_event, 0)); }
-    CafeHot hot(int t) const { CafeHot h; h.list = hot_list[t]; h.count = hot_count[t]; h.flag = hot_flag[t]; h.cap2 = hot_nb[t]; return h; }
+    CafeHot hot(int t) const { CafeHot h; h.list = hot_list[t]; h.count = count_of(t); h.flag = hot_flag[t]; h.cap2 = hot_nb[t]; return h; }
     // buckets a warp of a sparse launch scans, in units of 32: enough warps to fill the GPU first, long scans second
     static int scan_its(int nb, int most) {
         const int its = (int)((nb + 148 * 16 * 32 - 1) / (148 * 16 * 32));
@@ -2058,10 +2090,28 @@ struct CudaBackend {
     // that outnumber the LRU buckets 256 times go by the compacted lists, which only the launches have.
     bool run_job(const CafeJob& J0, uint8_t* const marks[2], uint32_t* ring, double refit_above, int real_n, bool adjust,
                  int round_cap, CafeJobOutcome* out) {
-        if (job_blocks < 1 || cafe_prof_serialise() || J0.M > CAFE_JOB_MOST || (int64_t)J0.M >= 256 * (int64_t)J0.n2) return false;
+        sort_join(0);
+        if (!carries(J0.M, J0.n2)) {
+            if (find_pending) {   // (timing was switched on since the sort)
+                find_now(stream);
+                if (gather_imp) gather_counts(gather_imp, J0.ord1, J0.ord2, J0.M, gather_simp1, gather_simp2);
+                gather_imp = nullptr;
+            }
+            return false;
+        }
         CafeJob J = J0;
         J.memo1 = memo1;
         CafeJobRun P;
+        P.first_of_call = find_pending ? 1 : 0;
+        if (find_pending) {
+            find_pending = false;
+            gather_imp = nullptr;
+            hot_set ^= 1;
+            find[0].count = count_of(0); find[1].count = count_of(1);
+        }
+        P.find[0] = find[0]; P.find[1] = find[1];
+        P.other_count = hot_counts + 4 * (hot_set ^ 1);
+        P.simp1 = const_cast<float*>(J.simp1); P.simp2 = const_cast<float*>(J.simp2);
         P.hot1 = hot(0); P.hot2 = hot(1);
         P.beg1 = const_cast<int32_t*>(J.beg1); P.beg2 = const_cast<int32_t*>(J.beg2);
         P.marks[0] = marks[0]; P.marks[1] = marks[1];
@@ -2072,7 +2122,6 @@ struct CudaBackend {
         P.units = std::min(CAFE_SCAN_MAIN / 32, std::max(1, cafe_blocks(J.n1, 32 * blocks * (CAFE_JOB_THREADS / 32))));
         P.ticket = job_ticket = job_ticket == INT32_MAX ? 1 : job_ticket + 1;
         void* args[] = {&J, &P};
-        sort_join(0);
         {
             CAFE_PROF(CAFE_P_MAIN, stream);
             check(cudaLaunchCooperativeKernel((const void*)k_whole_job, dim3((unsigned)blocks), dim3(CAFE_JOB_THREADS), args, 0, stream));
