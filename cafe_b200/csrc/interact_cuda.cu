@@ -121,9 +121,9 @@ struct CafeInteract {
     int blocks_of_rows;                    // ceil(nv / CAFE_IT_EDGE)
 };
 
-// the vectors of samples [b0, b0 + ns), back to back
+// the vectors of samples [b0, b0 + ns), one every `pitch` floats
 template <int DD>
-__device__ __forceinline__ void cafe_interact_stage(const CafeInteract& P, int64_t b0, int ns, float* T) {
+__device__ __forceinline__ void cafe_interact_stage(const CafeInteract& P, int64_t b0, int ns, float* T, const int pitch) {
     const int D = DD ? DD : P.D;
     const int q = (threadIdx.x & ((1 << P.lane_shift) - 1)) * 4, step = blockDim.x >> P.lane_shift;
     if (q >= D) return;
@@ -133,34 +133,40 @@ __device__ __forceinline__ void cafe_interact_stage(const CafeInteract& P, int64
         while (v >= P.nv) { v -= P.nv; ++s; }
         const int64_t b = b0 + s;
         const float* src = v < lead ? P.x + b * D : P.emb + b * P.sample_stride + (int64_t)(v - lead) * P.field_stride;
-        cafe_cp16(T + r * D + q, src + q);
+        cafe_cp16(T + r * pitch + q, src + q);
     }
 }
 
 // Forward.  The pairs of a sample are tiles of 7 x 7 vectors on and below the diagonal.  KL neighbouring lanes share a
-// tile and take every KL-th 16-byte piece of its vectors: 14 loads from shared memory feed 196 multiply-adds, and the
-// eight lanes of a load phase read 128 consecutive bytes.  The lanes' partial sums are added in a halving exchange that
-// leaves one (KL = 8) or two (KL = 4) rows of the tile with every lane.
+// tile and take every KL-th 16-byte piece of its vectors, four pieces each: 14 loads from shared memory feed 196
+// multiply-adds.  The lanes' partial sums are added in a halving exchange that leaves 8 / KL rows of the tile with every lane;
+// the kernel is bound by instruction issue (67 % of the slots, the multiply-adds 30 % of the pipe), and with fewer pieces per
+// lane the exchange is as long as the sums.  65 536 samples of 27 vectors: D 64 254 us (525 a sample per block, a float per load;
+// 285 with eight lanes a tile), D 32 149 (339; 199), D 16 98 (250; 127); 29 000 of D 128 193 us (419) = 2.4 TB/s.  Double
+// multiply-adds (f32x2) halve the instructions but take 166 registers and were no faster at D 64, slower at D 128.
+// The vectors lie at a pitch that puts the pieces which the tiles of a load phase (eight lanes) read, 7 vectors apart, into
+// different banks.
+template <int DD, int KL> __host__ __device__ constexpr int cafe_interact_pitch(int D) { return KL == 1 ? D + 4 : KL == 2 ? D + 8 : KL == 4 ? D + 16 : D; }
 template <int DD, int KL>
 __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_forward_tiled(const CafeInteract P, float* __restrict__ out, int64_t out_stride) {
     extern __shared__ __align__(16) float sh[];
     constexpr int E = CAFE_IT_EDGE, N = 8 * E;
-    const int D = DD ? DD : P.D;
-    const int group = P.per_group * P.nv * D;
-    float* Z = sh + 2 * group + (E - 1) * D;   // (tiles read up to E - 1 vectors past the last one)
+    const int D = DD ? DD : P.D, pitch = cafe_interact_pitch<DD, KL>(D);
+    const int group = P.per_group * P.nv * pitch;
+    float* Z = sh + 2 * group + (E - 1) * pitch;   // (tiles read up to E - 1 vectors past the last one)
     const int tiles = P.blocks_of_rows * (P.blocks_of_rows + 1) / 2;
     const int slots = blockDim.x / KL, slot = threadIdx.x / KL, kl = threadIdx.x % KL;
     const int lead = P.x ? D : 0;
     const int64_t step = (int64_t)gridDim.x * P.per_group;
     int64_t b0 = (int64_t)blockIdx.x * P.per_group;
-    cafe_interact_stage<DD>(P, b0, (int)min((int64_t)P.per_group, P.B - b0), sh);
+    cafe_interact_stage<DD>(P, b0, (int)min((int64_t)P.per_group, P.B - b0), sh, pitch);
     cafe_cp_commit();
     for (int half = 0; b0 < P.B; b0 += step, half ^= 1) {
         const int ns = (int)min((int64_t)P.per_group, P.B - b0);
         const float* T = sh + half * group;
         cafe_cp_wait();
         __syncthreads();   // this group has arrived; everyone is done with the other half and with Z
-        if (b0 + step < P.B) cafe_interact_stage<DD>(P, b0 + step, (int)min((int64_t)P.per_group, P.B - b0 - step), sh + (half ^ 1) * group);
+        if (b0 + step < P.B) cafe_interact_stage<DD>(P, b0 + step, (int)min((int64_t)P.per_group, P.B - b0 - step), sh + (half ^ 1) * group, pitch);
         cafe_cp_commit();
         for (int t0 = 0; t0 < ns * tiles; t0 += slots) {
             const int t = min(t0 + slot, ns * tiles - 1);   // (spare lanes repeat the last tile and write nothing)
@@ -168,8 +174,8 @@ __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_forward_tiled(c
             int bi = 0;
             while ((bi + 1) * (bi + 2) / 2 <= tile) ++bi;
             const int bj = tile - bi * (bi + 1) / 2;
-            const float* A = T + (s * P.nv + bi * E) * D;
-            const float* C = T + (s * P.nv + bj * E) * D;
+            const float* A = T + (s * P.nv + bi * E) * pitch;
+            const float* C = T + (s * P.nv + bj * E) * pitch;
             float acc[N];
 #pragma unroll
             for (int i = 0; i < N; ++i) acc[i] = 0.f;
@@ -177,10 +183,10 @@ __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_forward_tiled(c
             for (int q = kl * 4; q < D; q += KL * 4) {
                 float4 a[E];
 #pragma unroll
-                for (int r = 0; r < E; ++r) a[r] = *reinterpret_cast<const float4*>(A + r * D + q);
+                for (int r = 0; r < E; ++r) a[r] = *reinterpret_cast<const float4*>(A + r * pitch + q);
 #pragma unroll
                 for (int c = 0; c < E; ++c) {
-                    const float4 w = *reinterpret_cast<const float4*>(C + c * D + q);
+                    const float4 w = *reinterpret_cast<const float4*>(C + c * pitch + q);
 #pragma unroll
                     for (int r = 0; r < E; ++r) {
                         float v = acc[r * E + c];
@@ -206,9 +212,10 @@ __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_forward_tiled(c
                 for (int h = 0; h < RL; ++h) {
                     const int r = kl * RL + h, i = bi * E + r;
                     if (r < E && i < P.nv) {
-                        float* z = Z + s * P.npairs + cafe_pair_index(i, 0, P.off);
+                        float* z = Z + s * P.npairs + cafe_pair_index(i, 0, P.off) + bj * E;
+                        const int n = i + P.off - bj * E;   // columns of the row that count
 #pragma unroll
-                        for (int c = 0; c < E; ++c) if (bj * E + c < i + P.off) z[bj * E + c] = acc[h * E + c];
+                        for (int c = 0; c < E; ++c) if (c < n) z[c] = acc[h * E + c];
                     }
                 }
             }
@@ -216,7 +223,7 @@ __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_forward_tiled(c
         __syncthreads();
         for (int s = 0; s < ns; ++s) {
             float* o = out + (b0 + s) * out_stride;
-            for (int e = threadIdx.x; e < P.width; e += blockDim.x) o[e] = e < lead ? T[s * P.nv * D + e] : Z[s * P.npairs + e - lead];
+            for (int e = threadIdx.x; e < P.width; e += blockDim.x) o[e] = e < lead ? T[s * P.nv * pitch + e] : Z[s * P.npairs + e - lead];
         }
     }
 }
@@ -224,6 +231,8 @@ __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_forward_tiled(c
 // Backward.  The incoming row of a sample is spread into its symmetric weight matrix, rows padded to eight columns per
 // block of seven; a thread makes one 16-byte piece of seven gradient vectors, so that one piece of a vector (its lanes
 // read consecutive pieces) and two broadcast pieces of weights feed 28 multiply-adds.  Vectors are added in ascending order.
+// Bound by instruction issue too (75 %).  65 536 samples of 27 vectors: D 64 280 us (1052 with one output per thread and turn),
+// D 32 176 (591), D 16 141 (371); 29 000 of D 128 227 us (893) = 3.8 TB/s.
 template <int DD>
 __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_backward_tiled(const CafeInteract P, const float* __restrict__ grad_out,
                                                                              int64_t out_stride, float* __restrict__ grad_x,
@@ -244,7 +253,7 @@ __global__ void __launch_bounds__(CAFE_IT_THREADS, 2) k_interact_backward_tiled(
     int64_t b0 = (int64_t)blockIdx.x * P.per_group;
     auto fetch = [&](int64_t b, int half) {
         const int ns = (int)min((int64_t)P.per_group, P.B - b);
-        cafe_interact_stage<DD>(P, b, ns, sh + half * group);
+        cafe_interact_stage<DD>(P, b, ns, sh + half * group, D);
         for (int s = 0; s < ns; ++s)
             for (int e = threadIdx.x; e < P.width; e += blockDim.x)
                 cafe_cp4(raw + half * rows + s * P.width + e, grad_out + (b + s) * out_stride + e);
@@ -321,10 +330,12 @@ static void interact_plan(CafeInteract* P, const float* x, const float* emb, int
     P->lane_shift = 0;
     while ((4 << P->lane_shift) < D) ++P->lane_shift;
 }
-// Threads and samples per group for `lanes` threads of work per sample: about `want` threads a block, but no more samples
-// than leave every SM `resident` blocks to work on.
-static int interact_group(CafeInteract* P, int lanes, int want, int resident) {
+// Threads and samples per group for `lanes` threads of work and `bytes` of shared memory per sample: about `want` threads a
+// block, but no more samples than leave every SM `resident` blocks to work on, and room for them.
+static int interact_group(CafeInteract* P, int lanes, size_t bytes, int want, int resident) {
     int s = want / lanes;
+    const int room = (int)(224 * 1024 / resident / bytes);
+    if (s > room) s = room;
     const int fair = (P->B + CAFE_SMS * resident - 1) / (CAFE_SMS * resident);
     s = s < 1 ? 1 : (s > fair ? fair : s);
     P->per_group = s;
@@ -373,17 +384,16 @@ int cafe_dot_interaction_forward(const float* x_dev, const float* emb_dev, int64
     if (D % 4 == 0 && interact_pieces_ok(emb_dev, field_stride, sample_stride) && interact_pieces_ok(x_dev, 0, 0)) {
         CafeInteract P;
         interact_plan(&P, x_dev, emb_dev, field_stride, sample_stride, B, F, D, itself);
-        const int lanes = P.blocks_of_rows * (P.blocks_of_rows + 1) / 2 * (D < 32 ? 4 : 8);
-        const int threads = interact_group(&P, lanes, 240, 3);
-        const size_t sm = sizeof(float) * ((size_t)(2 * P.per_group * nv + CAFE_IT_EDGE - 1) * D + (size_t)P.per_group * npairs);
-        unsigned grid = 1;
+        const int tiles = P.blocks_of_rows * (P.blocks_of_rows + 1) / 2;
         cudaError_t e = cudaSuccess;
-        INTERACT_DISPATCH(D, constexpr int KL = DD == 16 ? 4 : 8; if (D >= 32 || DD == 16) {
+        INTERACT_DISPATCH(D, {
+            constexpr int KL = DD == 16 ? 1 : DD == 32 ? 2 : DD == 64 ? 4 : 8;
+            const int pitch = cafe_interact_pitch<DD, KL>(D);
+            const int threads = interact_group(&P, tiles * KL, sizeof(float) * (2 * (size_t)nv * pitch + npairs), KL == 8 ? 240 : 128, 3);
+            const size_t sm = sizeof(float) * ((size_t)(2 * P.per_group * nv + CAFE_IT_EDGE - 1) * pitch + (size_t)P.per_group * npairs);
+            unsigned grid = 1;
             e = interact_grid(k_interact_forward_tiled<DD, KL>, P, threads, 512, sm, &grid);
             if (e == cudaSuccess) k_interact_forward_tiled<DD, KL><<<grid, threads, sm, (cudaStream_t)stream>>>(P, out_dev, out_stride);
-        } else {
-            e = interact_grid(k_interact_forward_tiled<0, 4>, P, threads, 512, sm, &grid);
-            if (e == cudaSuccess) k_interact_forward_tiled<0, 4><<<grid, threads, sm, (cudaStream_t)stream>>>(P, out_dev, out_stride);
         });
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) { cafe_internal_set_error(cudaGetErrorString(e)); return CAFE_ERR_CUDA; }
@@ -409,7 +419,8 @@ int cafe_dot_interaction_backward(const float* x_dev, const float* emb_dev, int6
         interact_pieces_ok(grad_emb_dev, gfield_stride, gsample_stride) && interact_pieces_ok(grad_x_dev, 0, 0)) {
         CafeInteract P;
         interact_plan(&P, x_dev, emb_dev, field_stride, sample_stride, B, F, D, itself);
-        const int threads = interact_group(&P, P.blocks_of_rows << P.lane_shift, 128, 5);
+        const int threads = interact_group(&P, P.blocks_of_rows << P.lane_shift,
+                                           sizeof(float) * (size_t)(2 * (nv * D + P.width) + nv * (P.blocks_of_rows * 8 + 4)), 128, 4);
         const size_t sm = sizeof(float) * ((size_t)P.per_group * (2 * (nv * D + P.width) + nv * (P.blocks_of_rows * 8 + 4)) + P.npairs);
         unsigned grid = 1;
         cudaError_t e = cudaSuccess;
