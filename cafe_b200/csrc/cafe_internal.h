@@ -27,11 +27,12 @@ struct CafeEmbedWorkspace {
     int32_t* mask = nullptr;     // [cap] newly-hot flag per lookup
     int32_t* post_row = nullptr; // [cap] hot row after the lookup's own call
     uint32_t* key = nullptr;                 // [cap] unified row key of every lookup
+    uint32_t* sort_id = nullptr;             // [cap] id of every lookup, for the bucket sorts
     uint2* rows = nullptr;                   // [cap] (row key, position) sorted by row
     float* partial = nullptr;    // [2 * chunks * CAFE_MAX_DIM] partial row sums of chunk-spanning rows
     int32_t* row_winner = nullptr;   // [hotn] migration: highest position that claims a hot row in this call (-1 between calls)
     uint2* rows_tmp = nullptr;       // [cap] pairs between two passes of the row sort
-    const uint32_t* keys_of = nullptr;   // `key` was left by cafe_embed_resolve for the lookups whose global ids are in this array
+    const uint32_t* keys_of = nullptr;   // `key` and `sort_id` were left by cafe_embed_resolve for the lookups whose global ids are in this array
     int keys_total = 0;
     int32_t* sort_scratch = nullptr; // radix-sort histograms
     cudaStream_t late = nullptr;     // importance of fields whose gradients arrive behind a gate
@@ -50,9 +51,10 @@ CafeEmbedWorkspace* cafe_internal_ws(void* h);
 // use_presort: the last cafe_internal_presort was for exactly these ids (and they have not changed since)
 int cafe_internal_insert(void* h, const uint32_t* gid, const float* imp, const int* seg_off, int nseg, int32_t* mask,
                          int32_t* post_row, int mode, bool use_presort, cudaStream_t stream);
-// starts the insert's bucket sorts of `gid` beside whatever the caller queues next on `stream`
-// (also: a further sort to run with them, or null).  A null gid withdraws an earlier presort.
-void cafe_internal_presort(void* h, const uint32_t* gid, int n, const CafeSortDesc* also, cudaStream_t stream);
+// starts the bucket sorts for an insert of `gid` beside whatever the caller queues next on `stream`.  `ids` holds the same
+// ids in memory that stays as it is until the sorts are done (also: a further sort to run with them, or null).  A null gid
+// withdraws an earlier presort.
+void cafe_internal_presort(void* h, const uint32_t* gid, const uint32_t* ids, int n, const CafeSortDesc* also, cudaStream_t stream);
 // makes `stream` wait for sorts that a presort started: before their inputs are written again (they stay outstanding for
 // the call that uses them), or to use them
 int cafe_internal_sort_wait(void* h, cudaStream_t stream);

@@ -103,15 +103,16 @@ __device__ __forceinline__ uint32_t cafe_row_key(const CafeFields& F, int32_t co
     return code < 0 ? (uint32_t)((-code) % F.hotn) : (uint32_t)(F.hotn + F.hash_base[f] + code);
 }
 
-// The forward in two kernels, for training: k_embed_resolve does the sketch probe only (global id, row code, and the
-// unified row that the backward sorts by), k_embed_gather copies the rows named by the codes.
+// The forward in two kernels, for training: k_embed_resolve does the sketch probe only (global id, row code, and into arrays
+// of the library the two things that the backward sorts by: the id again and the unified row), k_embed_gather copies the
+// rows named by the codes.
 // Between the two the caller can start the backward's sorts, which need nothing but the first kernel's
 // outputs, so that they run beside the gather instead of after it.
 template <typename IdT>
 __global__ void __launch_bounds__(256)
 k_embed_resolve(const __grid_constant__ CafeFields F, const IdT* __restrict__ ids, const CafeMainBucket* __restrict__ mb,
-                const CafeMod n1, uint32_t* __restrict__ gid_out, int32_t* __restrict__ row_out, uint32_t* __restrict__ rowkey_out,
-                int total) {
+                const CafeMod n1, uint32_t* __restrict__ gid_out, int32_t* __restrict__ row_out, uint32_t* __restrict__ sort_id_out,
+                uint32_t* __restrict__ rowkey_out, int total) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= total) return;
     const int f = p / F.B;
@@ -127,7 +128,7 @@ k_embed_resolve(const __grid_constant__ CafeFields F, const IdT* __restrict__ id
     gid_out[p] = x;
     const int32_t code = r ? -r : (int32_t)(x % (uint32_t)F.hash_size[f]);
     row_out[p] = code;
-    if (rowkey_out) rowkey_out[p] = cafe_row_key(F, code, f);
+    if (rowkey_out) { sort_id_out[p] = x; rowkey_out[p] = cafe_row_key(F, code, f); }
 }
 
 template <int G>
@@ -302,11 +303,13 @@ k_migrate(const __grid_constant__ CafeFields F, const IdT* __restrict__ ids, con
 // sums that a second kernel adds in chunk order.  The order of additions is fixed by the sort, so
 // results are deterministic.
 // ---------------------------------------------------------------------------------------------
-__global__ void k_row_keys(const __grid_constant__ CafeFields F, const int32_t* __restrict__ row, int total,
-                           uint32_t* __restrict__ key) {
+// (gid, sort_id: the ids too, for sorts that run beside the caller's work; or null)
+__global__ void k_row_keys(const __grid_constant__ CafeFields F, const int32_t* __restrict__ row, const uint32_t* __restrict__ gid,
+                           int total, uint32_t* __restrict__ key, uint32_t* __restrict__ sort_id) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= total) return;
     key[p] = cafe_row_key(F, row[p], p / F.B);
+    if (gid) sort_id[p] = gid[p];
 }
 
 __device__ __forceinline__ float* row_ptr(const CafeFields& F, uint32_t key, int pos) {
@@ -671,7 +674,7 @@ int cafe_embed_ws_init(CafeEmbedWorkspace* ws, int cap, int hotn) {
     auto A = [&](void** p, size_t n) { if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1); };
     A((void**)&ws->norm, 4 * M); A((void**)&ws->imp, 4 * M); A((void**)&ws->totals, 4 * CAFE_MAX_SEGMENTS);
     A((void**)&ws->mask, 4 * M); A((void**)&ws->post_row, 4 * M);
-    A((void**)&ws->key, 4 * M); A((void**)&ws->rows, sizeof(uint2) * M); A((void**)&ws->rows_tmp, sizeof(uint2) * M);
+    A((void**)&ws->key, 4 * M); A((void**)&ws->sort_id, 4 * M); A((void**)&ws->rows, sizeof(uint2) * M); A((void**)&ws->rows_tmp, sizeof(uint2) * M);
     A((void**)&ws->partial, sizeof(float) * 2 * chunks * CAFE_MAX_DIM);
     A((void**)&ws->row_winner, 4 * (size_t)(hotn > 0 ? hotn : 1));
     if (e == cudaSuccess) e = cudaMemset(ws->row_winner, 0xff, 4 * (size_t)(hotn > 0 ? hotn : 1));   // -1: unclaimed
@@ -683,7 +686,7 @@ int cafe_embed_ws_init(CafeEmbedWorkspace* ws, int cap, int hotn) {
 }
 
 void cafe_embed_ws_free(CafeEmbedWorkspace* ws) {
-    void* ptrs[] = {ws->norm, ws->imp, ws->totals, ws->mask, ws->post_row, ws->key, ws->rows,
+    void* ptrs[] = {ws->norm, ws->imp, ws->totals, ws->mask, ws->post_row, ws->key, ws->sort_id, ws->rows,
                     ws->rows_tmp, ws->partial, ws->sort_scratch, ws->row_winner};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (ws->late) { cudaStreamSynchronize(ws->late); cudaStreamDestroy(ws->late); }
@@ -822,22 +825,23 @@ int cafe_embed_resolve(void* h, const void* ids_dev, int ids_are_int64, int nfie
     if (hotn != V.lim) return CAFE_ERR_ARG;
     CafeEmbedWorkspace* ws = cafe_internal_ws(h);
     const int total = (int)total64;
-    // the row keys are kept for the backward when the lookups fit the workspace (and rows fit the unified numbering)
+    // ids and row keys are kept for the backward's sorts when the lookups fit the workspace (and rows fit the unified numbering)
     const bool keep = total <= ws->cap && rows + hotn <= 0x7fffffffLL;
     uint32_t* keys = keep ? ws->key : nullptr;
+    uint32_t* sort_id = keep ? ws->sort_id : nullptr;
     const CafeMod mod = cafe_mod_of(V.n1);
     forget_head_start(h, gid_out_dev, row_out_dev);
     ws->keys_of = keep ? gid_out_dev : nullptr;
     ws->keys_total = keep ? total : 0;
     cudaStream_t st = (cudaStream_t)stream;
-    if (keep) {   // sorts of an earlier forward may still be reading the keys
+    if (keep) {   // sorts of an earlier forward may still be reading them
         const int rc = cafe_internal_sort_wait(h, st);
         if (rc != CAFE_OK) return rc;
     }
     CAFE_PROF(CAFE_P_QUERY, st);
     const int blocks = (total + 255) / 256;
-    if (ids_are_int64) k_embed_resolve<int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, keys, total);
-    else k_embed_resolve<int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, keys, total);
+    if (ids_are_int64) k_embed_resolve<int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, sort_id, keys, total);
+    else k_embed_resolve<int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, sort_id, keys, total);
     return fail_cuda("cafe_embed_resolve");
 }
 
@@ -997,12 +1001,12 @@ static CafeSortDesc row_sort_desc(CafeEmbedWorkspace* ws, const CafeFields& F, i
     D.tmp = ws->rows_tmp; D.out = ws->rows; D.scratch = ws->sort_scratch;
     return D;
 }
-static void row_keys(CafeEmbedWorkspace* ws, const CafeFields& F, const int32_t* row_dev, int total, cudaStream_t st) {
+static void row_keys(CafeEmbedWorkspace* ws, const CafeFields& F, const int32_t* row_dev, const uint32_t* gid_dev, int total, cudaStream_t st) {
     CAFE_PROF(CAFE_P_ROWKEYS, st);
-    k_row_keys<<<(total + 255) / 256, 256, 0, st>>>(F, row_dev, total, ws->key);
+    k_row_keys<<<(total + 255) / 256, 256, 0, st>>>(F, row_dev, gid_dev, total, ws->key, ws->sort_id);
 }
 static int scatter_prepare(CafeEmbedWorkspace* ws, const CafeFields& F, const int32_t* row_dev, int total, cudaStream_t st) {
-    row_keys(ws, F, row_dev, total, st);
+    row_keys(ws, F, row_dev, nullptr, total, st);
     CAFE_PROF(CAFE_P_ROWSORT, st);
     CafeSortBatch B;
     B.count = 1;
@@ -1065,7 +1069,10 @@ int cafe_scatter_sgd(void* h, const float* grad_dev, int64_t field_stride, int64
 }
 
 // Starts (or recognises as already started by cafe_embed_backward_begin) the side work of one backward call: the row sort
-// of the scatter and the bucket sorts of the parallel insert, in one batch on a stream of the sketch's.
+// of the scatter and the bucket sorts of the parallel insert, in one batch on a stream of the sketch's.  The sorts outlive
+// the call, and the caller's arrays need not: a forward whose backward never comes frees them while the sorts run, and a
+// sort that reads its keys once to count them and once to place them would then place pairs outside its arrays.  So the
+// sorts read arrays of the library, which are written again only behind cafe_internal_sort_wait.
 static int backward_side_work(void* h, CafeEmbedWorkspace* ws, const CafeFields& FS, const uint32_t* gid_dev,
                               const int32_t* row_dev, int total, int insert_mode, cudaStream_t st) {
     // (row keys serve the lookups they were left for once: the arrays may be the caller's to rewrite afterwards)
@@ -1078,12 +1085,12 @@ static int backward_side_work(void* h, CafeEmbedWorkspace* ws, const CafeFields&
         if (rc != CAFE_OK) return rc;
     }
     if (insert_mode == CAFE_INSERT_SEQUENTIAL) { ws->keys_of = nullptr; return scatter_prepare(ws, FS, row_dev, total, st); }
-    // row keys left by cafe_embed_resolve for exactly these lookups
+    // ids and row keys left by cafe_embed_resolve for exactly these lookups
     const bool have = ws->keys_of == gid_dev && ws->keys_total == total;
     ws->keys_of = nullptr;
-    if (!have) row_keys(ws, FS, row_dev, total, st);
+    if (!have) row_keys(ws, FS, row_dev, gid_dev, total, st);
     const CafeSortDesc rows = row_sort_desc(ws, FS, total);
-    cafe_internal_presort(h, gid_dev, total, &rows, st);
+    cafe_internal_presort(h, gid_dev, ws->sort_id, total, &rows, st);
     return CAFE_OK;
 }
 
@@ -1142,7 +1149,7 @@ static int embed_backward_impl(void* h, const float* grad_dev, int64_t field_str
         if (rc == CAFE_OK) cafe_internal_set_gate(h, gate_field, ws->ev_late);
     }
     if (rc != CAFE_OK) {
-        cafe_internal_presort(h, nullptr, 0, nullptr, st);   // withdraws the sorts started above
+        cafe_internal_presort(h, nullptr, nullptr, 0, nullptr, st);   // withdraws the sorts started above
         return rc;
     }
     int seg[CAFE_MAX_SEGMENTS + 1];

@@ -2301,16 +2301,16 @@ int cafe_internal_insert(void* h, const uint32_t* gid, const float* imp, const i
                          int32_t* post_row, int mode, bool use_presort, cudaStream_t stream) {
     CafeHandle* H = (CafeHandle*)h;
     H->eng.be.stream = stream;
-    if (!use_presort) H->eng.presort(nullptr, 0);
+    if (!use_presort) H->eng.presort(nullptr, nullptr, 0);
     int rc = H->eng.insert_segments(gid, imp, seg_off, nseg, mask, post_row, mode != CAFE_INSERT_SEQUENTIAL);
     return finish(H, rc, "cafe_sketch_insert");
 }
-void cafe_internal_presort(void* h, const uint32_t* gid, int n, const CafeSortDesc* also, cudaStream_t stream) {
+void cafe_internal_presort(void* h, const uint32_t* gid, const uint32_t* ids, int n, const CafeSortDesc* also, cudaStream_t stream) {
     CafeHandle* H = (CafeHandle*)h;
     H->eng.be.stream = stream;
     H->eng.be.batch.count = 0;
     if (also && gid) H->eng.be.batch.d[H->eng.be.batch.count++] = *also;
-    H->eng.presort(gid, n);
+    H->eng.presort(gid, ids, n);
     H->eng.be.batch.count = 0;
 }
 int cafe_internal_sort_wait(void* h, cudaStream_t stream) {

@@ -153,13 +153,14 @@ public:
 
     // Starts the bucket sorts of the next insert_segments call early, on the backend's side lanes, for
     // a caller that knows the ids before it knows the counts.  Only honoured when that call passes the
-    // same pointer and its whole input is one stretch of n lookups.
-    void presort(const uint32_t* gid, int n) {
+    // same pointer and its whole input is one stretch of n lookups.  The sorts read `ids`, which holds
+    // the same values in memory that outlives them.
+    void presort(const uint32_t* gid, const uint32_t* ids, int n) {
         presorted_gid = nullptr;
         if (ready) be.sort_join(-1);   // a null gid withdraws an earlier presort
         if (!ready || !gid || n <= 0 || n > cap) return;
-        be.sort_lookups(gid, n, n2, ord2, sgid2, start2, beg2, 2);
-        be.sort_lookups(gid, n, n1, ord1, sgid1, start1, beg1, 1);
+        be.sort_lookups(ids, n, n2, ord2, sgid2, start2, beg2, 2);
+        be.sort_lookups(ids, n, n1, ord1, sgid1, start1, beg1, 1);
         presorted_gid = gid; presorted_n = n;
     }
 

@@ -369,3 +369,48 @@ def test_a_dropped_forward_leaves_nothing_behind():
         np.testing.assert_allclose(grp.weight_high.detach().cpu().numpy(), orc.wh, rtol=1e-5, atol=1e-7)
         for f in range(2):
             np.testing.assert_allclose(grp.weight_hash[f].detach().cpu().numpy(), orc.wc[f], rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("B", [20_000, 70_000])
+def test_a_dropped_forwards_sorts_survive_its_buffers(B):
+    """The head start of a forward whose backward never comes is still sorting when its id and row arrays are written again, by
+    the next forward or by whatever got their memory.  In the forms of the sort that read their keys twice (several tiles per
+    block of a cluster, a launch per step), at a call as large as the workspace.  The next batch's step must be that of a
+    group which never dropped a forward and inserts one lookup at a time."""
+    import torch
+    import cafe_b200
+    from cafe_b200 import _lib
+    from cafe_b200.sketch import _stream
+    cards, D, lib = [30_000, 2_000_000], 16, _lib.load()
+    a, b = (cafe_b200.SKEmbeddingGroup(cards, D, 0.02, 0.3, 1, 1, 1.0000005, device="cuda", max_batch=B, lr=0.1, seed=4, insert_mode=m)
+            for m in (cafe_b200.INSERT_PARALLEL, cafe_b200.INSERT_SEQUENTIAL))
+    assert a.sketch.capacity == 2 * B
+    fs = a._fields
+    gid, row = (torch.empty(2 * B, dtype=torch.int32, device="cuda") for _ in range(2))
+    out = torch.empty(B, 2, D, device="cuda")
+    rng = np.random.default_rng(B)
+    for step in range(4):
+        dropped = torch.from_numpy(np.stack([rng.integers(0, n, B) for n in cards])).cuda()
+        ids = torch.from_numpy(np.stack([np.minimum(rng.zipf(1.3, B) - 1, n - 1) for n in cards])).cuda()
+        g = torch.from_numpy((rng.standard_normal((B, 2, D)) * 0.01).astype(np.float32)).cuda()
+        junk = torch.from_numpy(rng.integers(-2**31, 2**31, 2 * B).astype(np.int32)).cuda()
+        wp, hp = fs.ptrs()
+        torch.cuda.synchronize()
+        st = _stream()
+        _lib.check(lib.cafe_embed_resolve(a.sketch.handle, dropped.data_ptr(), 1, 2, B, fs.f_offset, fs.hash_size, a.hotn,
+                                          gid.data_ptr(), row.data_ptr(), st), "resolve")
+        _lib.check(lib.cafe_embed_backward_begin(a.sketch.handle, gid.data_ptr(), row.data_ptr(), 2, B, fs.hash_size, wp, hp,
+                                                 a.hotn, D, a.insert_mode, st), "begin")
+        if step % 2:
+            gid.copy_(junk)
+            row.copy_(junk)
+        _lib.check(lib.cafe_embed_forward(a.sketch.handle, ids.data_ptr(), 1, 2, B, fs.f_offset, fs.hash_size, wp, hp, a.hotn, D,
+                                          out.data_ptr(), D, 2 * D, gid.data_ptr(), row.data_ptr(), st), "forward")
+        fs.backward(g, D, 2 * D, ids.reshape(-1), gid, row, B, a.lr, a.insert_mode)
+        want = b(ids)
+        assert torch.equal(out, want), f"step {step}: rows"
+        want.backward(g)
+        assert states_equal(a.sketch.state(), b.sketch.state()) == [], f"step {step}: sketch state"
+        assert torch.equal(a.weight_high, b.weight_high), f"step {step}: hot table"
+        for f in range(2):
+            assert torch.equal(a.weight_hash[f], b.weight_hash[f]), f"step {step}: hash table {f}"
