@@ -32,12 +32,10 @@ struct CafeEmbedWorkspace {
     float* partial = nullptr;    // [2 * chunks * CAFE_MAX_DIM] partial row sums of chunk-spanning rows
     int32_t* row_winner = nullptr;   // [hotn] migration: highest position that claims a hot row in this call (-1 between calls)
     uint2* rows_tmp = nullptr;       // [cap] pairs between two passes of the row sort
-    const uint32_t* keys_of = nullptr;   // `key` and `sort_id` were left by cafe_embed_resolve for the lookups whose global ids are in this array
-    int keys_total = 0;
     int32_t* sort_scratch = nullptr; // radix-sort histograms
     cudaStream_t late = nullptr;     // importance of fields whose gradients arrive behind a gate
     cudaEvent_t ev_late = nullptr;
-    // arrays whose side work cafe_embed_backward_begin has already started (null: none)
+    // arrays whose side work a head start has already started (null: none)
     const uint32_t* begun_gid = nullptr;
     const int32_t* begun_row = nullptr;
     int begun_total = 0, begun_mode = 0;

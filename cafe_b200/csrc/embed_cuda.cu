@@ -103,11 +103,11 @@ __device__ __forceinline__ uint32_t cafe_row_key(const CafeFields& F, int32_t co
     return code < 0 ? (uint32_t)((-code) % F.hotn) : (uint32_t)(F.hotn + F.hash_base[f] + code);
 }
 
-// The forward in two kernels, for training: k_embed_resolve does the sketch probe only (global id, row code, and into arrays
-// of the library the two things that the backward sorts by: the id again and the unified row), k_embed_gather copies the
-// rows named by the codes.
-// Between the two the caller can start the backward's sorts, which need nothing but the first kernel's
-// outputs, so that they run beside the gather instead of after it.
+// The forward in two kernels, for training: k_embed_resolve does the sketch probe only (global id, row code, and, where the
+// backward's sorts follow at once, into arrays of the library the two things that they sort by: the id again and the unified
+// row), k_embed_gather copies the rows named by the codes.
+// The backward's sorts, which need nothing but the first kernel's outputs, start between the two, so that they run beside
+// the gather instead of after it.
 template <typename IdT>
 __global__ void __launch_bounds__(256)
 k_embed_resolve(const __grid_constant__ CafeFields F, const IdT* __restrict__ ids, const CafeMainBucket* __restrict__ mb,
@@ -740,12 +740,11 @@ static bool strides_ok(const float* p, int64_t fs, int64_t ss) { return aligned1
         default: { constexpr int G = 32; __VA_ARGS__; } break; \
     }
 
-// A forward has (re)written these two arrays: a head start or row keys left for arrays at the same addresses (of a
-// forward whose backward never came) belong to other lookups.
+// A forward has (re)written these two arrays: a head start for arrays at the same addresses (of a forward whose backward
+// never came) belongs to other lookups.
 static void forget_head_start(void* h, const uint32_t* gid, const int32_t* row) {
     CafeEmbedWorkspace* ws = cafe_internal_ws(h);
     if (ws->begun_gid == gid || ws->begun_row == row) { ws->begun_gid = nullptr; ws->begun_row = nullptr; ws->begun_total = 0; }
-    if (ws->keys_of == gid) ws->keys_of = nullptr;
 }
 
 static int launch_forward(const CafeFields& F, const void* ids_dev, int ids_are_int64, const CafeSketchView& V,
@@ -805,6 +804,19 @@ int cafe_records_to_batch(const int32_t* sparse_rows_dev, int B, int F, void* id
     return fail_cuda("cafe_records_to_batch");
 }
 
+// sort_id, keys: what a head start sorts by (see k_row_keys), or null
+static int launch_resolve(void* h, const CafeFields& F, const void* ids_dev, int ids_are_int64, uint32_t* gid_out_dev, int32_t* row_out_dev,
+                          uint32_t* sort_id, uint32_t* keys, int total, cudaStream_t st) {
+    const CafeSketchView V = cafe_internal_view(h);
+    const CafeMod mod = cafe_mod_of(V.n1);
+    forget_head_start(h, gid_out_dev, row_out_dev);
+    CAFE_PROF(CAFE_P_QUERY, st);
+    const int blocks = (total + 255) / 256;
+    if (ids_are_int64) k_embed_resolve<int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, sort_id, keys, total);
+    else k_embed_resolve<int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, sort_id, keys, total);
+    return fail_cuda("cafe_embed_resolve");
+}
+
 int cafe_embed_resolve(void* h, const void* ids_dev, int ids_are_int64, int nfields, int B, const int64_t* f_offset,
                        const int32_t* hash_size, int hotn, uint32_t* gid_out_dev, int32_t* row_out_dev, void* stream) {
     if (!h || nfields < 1 || nfields > CAFE_MAX_SEGMENTS || B < 0 || !f_offset || !hash_size) return CAFE_ERR_ARG;
@@ -815,34 +827,12 @@ int cafe_embed_resolve(void* h, const void* ids_dev, int ids_are_int64, int nfie
     CafeFields F;
     memset(&F, 0, sizeof(F));
     F.nfields = nfields; F.B = B; F.hotn = hotn;
-    int64_t rows = 0;
     for (int f = 0; f < nfields; ++f) {
         if (hash_size[f] < 1) return CAFE_ERR_ARG;
-        F.f_offset[f] = (uint32_t)f_offset[f]; F.hash_size[f] = hash_size[f]; F.hash_base[f] = (int32_t)rows;
-        rows += hash_size[f];
+        F.f_offset[f] = (uint32_t)f_offset[f]; F.hash_size[f] = hash_size[f];
     }
-    CafeSketchView V = cafe_internal_view(h);
-    if (hotn != V.lim) return CAFE_ERR_ARG;
-    CafeEmbedWorkspace* ws = cafe_internal_ws(h);
-    const int total = (int)total64;
-    // ids and row keys are kept for the backward's sorts when the lookups fit the workspace (and rows fit the unified numbering)
-    const bool keep = total <= ws->cap && rows + hotn <= 0x7fffffffLL;
-    uint32_t* keys = keep ? ws->key : nullptr;
-    uint32_t* sort_id = keep ? ws->sort_id : nullptr;
-    const CafeMod mod = cafe_mod_of(V.n1);
-    forget_head_start(h, gid_out_dev, row_out_dev);
-    ws->keys_of = keep ? gid_out_dev : nullptr;
-    ws->keys_total = keep ? total : 0;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (keep) {   // sorts of an earlier forward may still be reading them
-        const int rc = cafe_internal_sort_wait(h, st);
-        if (rc != CAFE_OK) return rc;
-    }
-    CAFE_PROF(CAFE_P_QUERY, st);
-    const int blocks = (total + 255) / 256;
-    if (ids_are_int64) k_embed_resolve<int64_t><<<blocks, 256, 0, st>>>(F, (const int64_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, sort_id, keys, total);
-    else k_embed_resolve<int32_t><<<blocks, 256, 0, st>>>(F, (const int32_t*)ids_dev, V.main, mod, gid_out_dev, row_out_dev, sort_id, keys, total);
-    return fail_cuda("cafe_embed_resolve");
+    if (hotn != cafe_internal_view(h).lim) return CAFE_ERR_ARG;
+    return launch_resolve(h, F, ids_dev, ids_are_int64, gid_out_dev, row_out_dev, nullptr, nullptr, (int)total64, (cudaStream_t)stream);
 }
 
 static int gather_impl(void* h, const int32_t* row_dev, int nfields, int B, const int32_t* hash_size, float* const* weight_hash,
@@ -1058,9 +1048,7 @@ int cafe_scatter_sgd(void* h, const float* grad_dev, int64_t field_stride, int64
     if (total == 0) return CAFE_OK;
     CafeEmbedWorkspace* ws = cafe_internal_ws(h);
     cudaStream_t st = (cudaStream_t)stream;
-    // the row keys of an earlier cafe_embed_resolve and the row order of an earlier head start are overwritten
-    ws->keys_of = nullptr;
-    ws->begun_gid = nullptr;
+    ws->begun_gid = nullptr;   // the row order of an earlier head start is overwritten
     rc = cafe_internal_sort_wait(h, st);
     if (rc != CAFE_OK) return rc;
     rc = scatter_prepare(ws, F, row_dev, total, st);
@@ -1068,14 +1056,18 @@ int cafe_scatter_sgd(void* h, const float* grad_dev, int64_t field_stride, int64
     return scatter_apply(ws, F, grad_dev, field_stride, sample_stride, total, D, lr, st);
 }
 
-// Starts (or recognises as already started by cafe_embed_backward_begin) the side work of one backward call: the row sort
-// of the scatter and the bucket sorts of the parallel insert, in one batch on a stream of the sketch's.  The sorts outlive
-// the call, and the caller's arrays need not: a forward whose backward never comes frees them while the sorts run, and a
-// sort that reads its keys once to count them and once to place them would then place pairs outside its arrays.  So the
-// sorts read arrays of the library, which are written again only behind cafe_internal_sort_wait.
+// The sorts of one backward call: the row sort of the scatter and the bucket sorts of the parallel insert, in one batch on a
+// stream of the sketch's.  The sorts outlive the call, and the caller's arrays need not: a forward whose backward never comes
+// frees them while the sorts run, and a sort that reads its keys once to count them and once to place them would then place
+// pairs outside its arrays.  So the sorts read arrays of the library, which are written again only behind
+// cafe_internal_sort_wait.
+static void start_sorts(void* h, CafeEmbedWorkspace* ws, const CafeFields& FS, const uint32_t* gid_dev, int total, cudaStream_t st) {
+    const CafeSortDesc rows = row_sort_desc(ws, FS, total);
+    cafe_internal_presort(h, gid_dev, ws->sort_id, total, &rows, st);
+}
+// Starts (or recognises as already started by a head start) the side work of one backward call.
 static int backward_side_work(void* h, CafeEmbedWorkspace* ws, const CafeFields& FS, const uint32_t* gid_dev,
                               const int32_t* row_dev, int total, int insert_mode, cudaStream_t st) {
-    // (row keys serve the lookups they were left for once: the arrays may be the caller's to rewrite afterwards)
     const bool begun = ws->begun_gid == gid_dev && ws->begun_row == row_dev && ws->begun_total == total &&
                        ws->begun_mode == insert_mode && gid_dev != nullptr;
     ws->begun_gid = nullptr; ws->begun_row = nullptr; ws->begun_total = 0;
@@ -1084,13 +1076,9 @@ static int backward_side_work(void* h, CafeEmbedWorkspace* ws, const CafeFields&
         const int rc = cafe_internal_sort_wait(h, st);
         if (rc != CAFE_OK) return rc;
     }
-    if (insert_mode == CAFE_INSERT_SEQUENTIAL) { ws->keys_of = nullptr; return scatter_prepare(ws, FS, row_dev, total, st); }
-    // ids and row keys left by cafe_embed_resolve for exactly these lookups
-    const bool have = ws->keys_of == gid_dev && ws->keys_total == total;
-    ws->keys_of = nullptr;
-    if (!have) row_keys(ws, FS, row_dev, gid_dev, total, st);
-    const CafeSortDesc rows = row_sort_desc(ws, FS, total);
-    cafe_internal_presort(h, gid_dev, ws->sort_id, total, &rows, st);
+    if (insert_mode == CAFE_INSERT_SEQUENTIAL) return scatter_prepare(ws, FS, row_dev, total, st);
+    row_keys(ws, FS, row_dev, gid_dev, total, st);
+    start_sorts(h, ws, FS, gid_dev, total, st);
     return CAFE_OK;
 }
 
@@ -1253,23 +1241,50 @@ int cafe_shard_pull_importance(void* h, const float* const* grad_rank, int nrank
     return fail_cuda("cafe_shard_pull_importance");
 }
 
+static int begin_check(void* h, CafeFields* FS, const void* gid_dev, const void* row_dev, int nfields, int B, const int64_t* f_offset,
+                       const int32_t* hash_size, float* const* weight_hash, float* weight_high, int hotn, int D) {
+    if (!h || !gid_dev || !row_dev) return CAFE_ERR_ARG;
+    const int rc = fill_fields(FS, nfields, B, D, hotn, f_offset, hash_size, weight_hash, weight_high);
+    if (rc != CAFE_OK) return rc;
+    return (int64_t)nfields * B > cafe_internal_ws(h)->cap ? CAFE_ERR_CAPACITY : CAFE_OK;
+}
+static void begun(CafeEmbedWorkspace* ws, const uint32_t* gid_dev, const int32_t* row_dev, int total, int insert_mode) {
+    ws->begun_gid = gid_dev; ws->begun_row = row_dev; ws->begun_total = total; ws->begun_mode = insert_mode;
+}
+
 int cafe_embed_backward_begin(void* h, const uint32_t* gid_dev, const int32_t* row_dev, int nfields, int B,
                               const int32_t* hash_size, float* const* weight_hash, float* weight_high, int hotn, int D,
                               int insert_mode, void* stream) {
-    if (!h || !gid_dev || !row_dev) return CAFE_ERR_ARG;
-    CafeEmbedWorkspace* ws = cafe_internal_ws(h);
     CafeFields FS;
     int64_t zero_off[CAFE_MAX_SEGMENTS] = {0};
-    int rc = fill_fields(&FS, nfields, B, D, hotn, zero_off, hash_size, weight_hash, weight_high);
-    if (rc != CAFE_OK) return rc;
-    const int64_t total = (int64_t)nfields * B;
-    if (total > ws->cap) return CAFE_ERR_CAPACITY;
-    if (total == 0) return CAFE_OK;
+    int rc = begin_check(h, &FS, gid_dev, row_dev, nfields, B, zero_off, hash_size, weight_hash, weight_high, hotn, D);
+    if (rc != CAFE_OK || B == 0) return rc;
+    CafeEmbedWorkspace* ws = cafe_internal_ws(h);
     ws->begun_gid = nullptr;
-    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, (int)total, insert_mode, (cudaStream_t)stream);
+    rc = backward_side_work(h, ws, FS, gid_dev, row_dev, nfields * B, insert_mode, (cudaStream_t)stream);
+    if (rc == CAFE_OK) begun(ws, gid_dev, row_dev, nfields * B, insert_mode);
+    return rc;
+}
+
+int cafe_embed_resolve_begin(void* h, const void* ids_dev, int ids_are_int64, int nfields, int B, const int64_t* f_offset,
+                             const int32_t* hash_size, float* const* weight_hash, float* weight_high, int hotn, int D,
+                             uint32_t* gid_out_dev, int32_t* row_out_dev, int insert_mode, void* stream) {
+    CafeFields F;
+    if (B == 0 && h && nfields >= 1 && nfields <= CAFE_MAX_SEGMENTS) return CAFE_OK;
+    int rc = begin_check(h, &F, gid_out_dev, row_out_dev, nfields, B, f_offset, hash_size, weight_hash, weight_high, hotn, D);
     if (rc != CAFE_OK) return rc;
-    ws->begun_gid = gid_dev; ws->begun_row = row_dev; ws->begun_total = (int)total; ws->begun_mode = insert_mode;
-    return CAFE_OK;
+    if (!ids_dev || hotn != cafe_internal_view(h).lim) return CAFE_ERR_ARG;
+    CafeEmbedWorkspace* ws = cafe_internal_ws(h);
+    const int total = nfields * B;
+    cudaStream_t st = (cudaStream_t)stream;
+    rc = cafe_internal_sort_wait(h, st);   // sorts of an earlier forward may still be reading the two arrays
+    if (rc == CAFE_OK) rc = launch_resolve(h, F, ids_dev, ids_are_int64, gid_out_dev, row_out_dev, ws->sort_id, ws->key, total, st);
+    if (rc != CAFE_OK) return rc;
+    ws->begun_gid = nullptr;
+    if (insert_mode == CAFE_INSERT_SEQUENTIAL) rc = scatter_prepare(ws, F, row_out_dev, total, st);
+    else start_sorts(h, ws, F, gid_out_dev, total, st);
+    if (rc == CAFE_OK) begun(ws, gid_out_dev, row_out_dev, total, insert_mode);
+    return rc;
 }
 
 // cafe_embed_backward with the importance array already computed (by cafe_shard_pull_importance)

@@ -175,9 +175,7 @@ class _PeerFunction(torch.autograd.Function):
             if training:
                 # sketch probe, then the backward's sorts on the side streams, then the gather with the exchange as
                 # its epilogue: the sorts run beside the gather and the dense model
-                _lib.check(lib.cafe_embed_resolve(grp.sketch.handle, own.data_ptr(), 1, Fg, G * Bl, f.f_offset, f.hash_size,
-                                                  f.hotn, gid.data_ptr(), row.data_ptr(), _stream()), "cafe_embed_resolve")
-                f.backward_begin(gid, row, G * Bl, grp.insert_mode)
+                f.resolve_begin(own, gid, row, grp.insert_mode)
                 _lib.check(lib.cafe_embed_gather_sharded(grp.sketch.handle, row.data_ptr(), Fg, G * Bl, f.hash_size, wp, hp,
                                                          f.hotn, D, out_rank, G, Bl, D, Fg * D, _stream()),
                            "cafe_embed_gather_sharded")

@@ -106,10 +106,9 @@ class _FieldSet:
         gp, rp = gid.data_ptr(), row.data_ptr()
         with torch.cuda.device(ids.device):
             st = _stream()
-            _lib.check(lib.cafe_embed_resolve(sk.handle, ids.data_ptr(), int(ids.dtype == torch.int64), self.nf, B,
-                                              self.f_offset, self.hash_size, self.hotn, gp, rp, st), "cafe_embed_resolve")
-            _lib.check(lib.cafe_embed_backward_begin(sk.handle, gp, rp, self.nf, B, self.hash_size, wp, hp, self.hotn, self.dim,
-                                                     mode, st), "cafe_embed_backward_begin")
+            _lib.check(lib.cafe_embed_resolve_begin(sk.handle, ids.data_ptr(), int(ids.dtype == torch.int64), self.nf, B,
+                                                    self.f_offset, self.hash_size, wp, hp, self.hotn, self.dim, gp, rp, mode, st),
+                       "cafe_embed_resolve_begin")
             _lib.check(lib.cafe_embed_gather(sk.handle, rp, self.nf, B, self.hash_size, wp, hp, self.hotn, self.dim,
                                              out.data_ptr(), field_stride, sample_stride, st), "cafe_embed_gather")
         return gid, row
@@ -137,14 +136,15 @@ class _FieldSet:
                                                         row.data_ptr(), self.nf, B, self.hash_size, wp, hp, self.hotn,
                                                         self.dim, float(lr), _stream()), "cafe_scatter_sgd")
 
-    def backward_begin(self, gid, row, B, mode):
-        """Starts the part of the backward that needs only the forward's outputs (the bucket sorts of the
-        sketch insert and the row sort of the scatter) on the library's side streams."""
+    def resolve_begin(self, ids: torch.Tensor, gid: torch.Tensor, row: torch.Tensor, mode: int):
+        """resolve() into given arrays, and the start of the part of the backward that needs only its outputs (the bucket
+        sorts of the sketch insert and the row sort of the scatter) on the library's side stream."""
         wp, hp = self.ptrs()
-        with torch.cuda.device(gid.device):
-            _lib.check(self.sketch.lib.cafe_embed_backward_begin(
-                self.sketch.handle, gid.data_ptr(), row.data_ptr(), self.nf, B, self.hash_size, wp, hp, self.hotn,
-                self.dim, mode, _stream()), "cafe_embed_backward_begin")
+        with torch.cuda.device(ids.device):
+            _lib.check(self.sketch.lib.cafe_embed_resolve_begin(
+                self.sketch.handle, ids.data_ptr(), int(ids.dtype == torch.int64), self.nf, ids.numel() // self.nf, self.f_offset,
+                self.hash_size, wp, hp, self.hotn, self.dim, gid.data_ptr(), row.data_ptr(), mode, _stream()),
+                "cafe_embed_resolve_begin")
 
     def backward_gated(self, grad, field_stride, sample_stride, ids, gid, row, B, lr, mode, gate_field, gate_event):
         """backward() whose gradient rows of the fields from gate_field on are complete only once gate_event

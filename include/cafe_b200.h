@@ -106,10 +106,10 @@ int cafe_records_to_batch(const int32_t* sparse_rows_dev, int B, int F, void* id
                           const int32_t* label_dev, float* label_out_dev, void* stream);
 
 /* cafe_embed_forward in two calls, for training.  cafe_embed_resolve is the query part alone
- * (tricks/sk_embedding_bag.py:101-113: global ids and row codes; it also keeps each lookup's bucket numbers
- * for the insert's sorts), cafe_embed_gather the two embedding_bag gathers and the where (:131-150) from the
- * row codes.  Between the two a caller can issue cafe_embed_backward_begin, whose sorts then run beside the
- * gather.  Results are identical to cafe_embed_forward. */
+ * (tricks/sk_embedding_bag.py:101-113: global ids and row codes), cafe_embed_gather the two embedding_bag
+ * gathers and the where (:131-150) from the row codes.  Results are identical to cafe_embed_forward.
+ * cafe_embed_resolve_begin (below) in the first one's place also starts the backward's sorts, which then run
+ * beside the gather. */
 int cafe_embed_resolve(void* handle, const void* ids_dev, int ids_are_int64, int nfields, int B, const int64_t* f_offset,
                        const int32_t* hash_size, int hotn, uint32_t* gid_out_dev, int32_t* row_out_dev, void* stream);
 int cafe_embed_gather(void* handle, const int32_t* row_dev, int nfields, int B, const int32_t* hash_size,
@@ -158,11 +158,16 @@ int cafe_embed_backward(void* handle, const float* grad_dev, int64_t field_strid
  * forward's outputs (the bucket orders of the sketch insert, the row order of the scatter), so that
  * it runs beside whatever the caller queues on `stream` in between (the dense model, an exchange of
  * gradients).  The backward recognises the head start by the same gid_dev / row_dev / sizes /
- * insert_mode and otherwise does the work itself; the two arrays must not change in between.  No
+ * insert_mode and otherwise does the work itself; the two arrays must not change in between (a caller
+ * that drops the backward may free or rewrite them at once: the work reads copies).  No
  * counterpart in the reference, whose insert is one sequential loop (sketch.cpp:268-280). */
 int cafe_embed_backward_begin(void* handle, const uint32_t* gid_dev, const int32_t* row_dev, int nfields, int B,
                               const int32_t* hash_size, float* const* weight_hash, float* weight_high, int hotn, int D,
                               int insert_mode, void* stream);
+/* cafe_embed_resolve followed by cafe_embed_backward_begin for its outputs, in one call. */
+int cafe_embed_resolve_begin(void* handle, const void* ids_dev, int ids_are_int64, int nfields, int B, const int64_t* f_offset,
+                             const int32_t* hash_size, float* const* weight_hash, float* weight_high, int hotn, int D,
+                             uint32_t* gid_out_dev, int32_t* row_out_dev, int insert_mode, void* stream);
 
 /* ---- field-sharded exchange over peer memory (one node, up to 8 ranks) -----------------------------
  * No counterpart in the reference (single GPU; its --dist flags are never used, dlrm_s_pytorch.py:

@@ -414,3 +414,32 @@ def test_a_dropped_forwards_sorts_survive_its_buffers(B):
         assert torch.equal(a.weight_high, b.weight_high), f"step {step}: hot table"
         for f in range(2):
             assert torch.equal(a.weight_hash[f], b.weight_hash[f]), f"step {step}: hash table {f}"
+
+
+@pytest.mark.parametrize("same_array", [True, False])
+def test_the_backward_sorts_by_the_rows_it_is_given(same_array):
+    """Row codes of cafe_embed_resolve that the caller changes (in place, or in an array of its own) before the backward: the
+    scatter goes to the changed rows.  lr is 1 and gradients are small whole numbers, so sums are exact."""
+    import torch
+    import cafe_b200
+    cards, D, B = [3000, 50000], 16, 300
+    grp = cafe_b200.SKEmbeddingGroup(cards, D, 0.02, 0.3, 1, 1, 1.0000005, device="cuda", max_batch=B, lr=1.0, seed=4)
+    rng = np.random.default_rng(3)
+    fs = grp._fields
+    with torch.no_grad():
+        for w in grp.weight_hash:
+            w.zero_()
+    ids = torch.from_numpy(np.stack([rng.integers(0, n, B) for n in cards])).cuda().reshape(-1)
+    gid, row = fs.resolve(ids)
+    assert bool((row >= 0).all())                       # nothing is hot yet
+    shifted = torch.cat([(row[f * B:(f + 1) * B] + 1) % grp.hash_sizes[f] for f in range(2)])
+    if same_array:
+        row.copy_(shifted)
+    else:
+        row = shifted
+    g = torch.from_numpy(rng.integers(-3, 4, (B, 2, D)).astype(np.float32)).cuda()
+    fs.backward(g, D, 2 * D, ids, gid, row, B, 1.0, grp.insert_mode)
+    for f in range(2):
+        want = torch.zeros_like(grp.weight_hash[f])
+        want.index_add_(0, row[f * B:(f + 1) * B].long(), -g[:, f])
+        assert torch.equal(grp.weight_hash[f].detach(), want), f
