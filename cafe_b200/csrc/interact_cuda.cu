@@ -346,7 +346,9 @@ static int interact_group(CafeInteract* P, int lanes, size_t bytes, int want, in
 template <typename K>
 static cudaError_t interact_grid(K kernel, const CafeInteract& P, int threads, int sm_threads, size_t smem, unsigned* grid) {
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // (the limit belongs to the kernel, not to the launch, and threads share it: always the same value, the largest a block
+        // can have, or one thread's smaller call would lower it between another's setting and its launch)
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
     }
     const int by_threads = sm_threads / threads, by_memory = (int)((227 * 1024) / (smem + 1024));

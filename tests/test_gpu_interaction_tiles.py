@@ -68,3 +68,48 @@ def test_every_form_against_fp64(B, F, D, dense, itself, layout, shift):
     written = torch.zeros_like(gbuf)
     written[shift:].as_strided((B, F, D), (ss, fs, 1)).fill_(1.0)
     assert bool((gbuf[written == 0] == 3.0).all())      # nothing beside the rows
+
+
+@pytest.mark.parametrize("backward", [False, True])
+def test_threads_with_different_sizes(backward):
+    """Threads whose calls share a kernel but want different amounts of shared memory, all above the default limit: every call
+    is taken, and the results are those of the same calls made alone."""
+    import threading
+    import torch
+    from cafe_b200 import _lib
+    lib = _lib.load()
+    B, D, rounds, workers = 1, 128, 10_000, 8
+    calls, alone = [], []
+    for k in range(workers):
+        F = (50, 40)[k % 2] if backward else (62, 45)[k % 2]
+        gen = torch.Generator(device="cuda").manual_seed(k)
+        x, emb, g = (torch.randn(*s, device="cuda", generator=gen) for s in ((B, D), (B, F, D), (B, D + (F + 1) * F // 2)))
+        out = [torch.empty_like(x), torch.empty_like(emb)] if backward else [torch.empty_like(g)]
+        args = (x.data_ptr(), emb.data_ptr(), D, F * D, B, F, D, 0)
+        if backward:
+            fn, args = lib.cafe_dot_interaction_backward, args + (g.data_ptr(), g.shape[1], out[0].data_ptr(), out[1].data_ptr(), D, F * D)
+        else:
+            fn, args = lib.cafe_dot_interaction_forward, args + (out[0].data_ptr(), g.shape[1])
+        calls.append((fn, args, out, (x, emb, g)))
+        _lib.check(fn(*args, torch.cuda.current_stream().cuda_stream), "alone")
+        alone.append([t.clone() for t in out])
+        for t in out:
+            t.zero_()
+    torch.cuda.synchronize()
+    refused = [0] * workers
+
+    def work(k):
+        stream = torch.cuda.Stream()
+        fn, args, _, _ = calls[k]
+        for _ in range(rounds):
+            refused[k] += fn(*args, stream.cuda_stream) != _lib.OK
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(workers)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert refused == [0] * workers
+    for k in range(workers):
+        assert all(torch.equal(u, v) for u, v in zip(alone[k], calls[k][2]))
