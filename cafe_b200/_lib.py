@@ -38,6 +38,7 @@ SIGNATURES = {
     "cafe_sketch_set_scalars": (c_int, [_vp, _i64p, c_double]),
     "cafe_sketch_tuning": (c_int, [_vp, c_int, c_int]),
     "cafe_sketch_stats": (c_int, [_vp, _i64p]),
+    "cafe_sketch_one_launch_jobs": (c_int64, [_vp]),
     "cafe_sketch_dump": (c_int, [_vp, _u32p, _f32p, _i32p, _u8p, _u32p, _f32p, _i32p, _i32p, _u8p, _u32p, _vp]),
     "cafe_sketch_load": (c_int, [_vp, _u32p, _f32p, _i32p, _u8p, _u32p, _f32p, _i32p, _i32p, _u8p, _u32p, c_int, _vp]),
     "cafe_embed_forward": (c_int, [_vp, _vp, c_int, c_int, c_int, _i64p, _i32p, POINTER(_vp), _vp, c_int, c_int, _vp,

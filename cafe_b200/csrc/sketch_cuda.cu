@@ -1518,6 +1518,8 @@ __global__ void __launch_bounds__(128) k_lru_pass_compact(const __grid_constant_
 // (the timeline's steps take one position or op per thread there: a chain of dependent loads each, so four or eight in a row
 // per thread, as in the launches of their own, took 6 to 19 us a step)
 #define CAFE_JOB_RESIDENT 3      // blocks per SM (the list replay takes 168 registers)
+// (the scratch of the timeline's blocks, tl_blk and tl_agg, is sized for blocks of CAFE_TL_SMALL)
+static_assert(CAFE_JOB_THREADS >= CAFE_TL_SMALL && CAFE_TL_BLOCK >= CAFE_TL_SMALL, "timeline blocks smaller than their scratch allows for");
 
 enum { CAFE_JOB_DONE = 0, CAFE_JOB_ROUND_CAP = 1, CAFE_JOB_ERROR = 2, CAFE_JOB_EMPTY = 3 };
 struct CafeJobRun {
@@ -1850,6 +1852,7 @@ struct CudaBackend {
     CafeRoundResult* job_res = nullptr;   // [2] round results of the whole-job launch
     CafeJobOutcome* job_out = nullptr;    // what it reports, in host memory
     int32_t job_ticket = 0;
+    int64_t jobs_launched = 0;            // jobs that went by it
     int job_blocks = 0;                   // blocks of it that are resident at once (0: no cooperative launches here)
 
     ~CudaBackend() {
@@ -2156,6 +2159,7 @@ struct CudaBackend {
         {
             CAFE_PROF(CAFE_P_MAIN, stream);
             check(cudaLaunchCooperativeKernel((const void*)k_whole_job, dim3((unsigned)blocks), dim3(CAFE_JOB_THREADS), args, 0, stream));
+            ++jobs_launched;
         }
         // The record is written as soon as the rounds have converged; what the host queues next runs behind the rest of the
         // launch, where a wait for its end would leave the GPU idle while the host wakes up and launches (11 us: a Kaggle-shape
@@ -2437,6 +2441,11 @@ int cafe_sketch_tuning(void* h, int window, int round_cap) {
     if (window > 0) H->eng.window = window > CAFE_MAX_SEGMENTS ? CAFE_MAX_SEGMENTS : window;
     if (round_cap > 0) H->eng.round_cap = round_cap;
     return CAFE_OK;
+}
+
+int64_t cafe_sketch_one_launch_jobs(void* h) {
+    if (!h) return 0;
+    return ((CafeHandle*)h)->eng.be.jobs_launched;
 }
 
 int cafe_sketch_stats(void* h, int64_t* out13) {

@@ -136,6 +136,10 @@ class HotSketch:
         self.lib.cafe_sketch_stats(self.handle, _np_ptr(s, _lib._i64p))
         return dict(zip(STAT_NAMES, (int(x) for x in s)))
 
+    def one_launch_jobs(self) -> int:
+        """How many of stats()["jobs"] ran in one launch each."""
+        return int(self.lib.cafe_sketch_one_launch_jobs(self.handle))
+
     def state(self) -> dict:
         """Whole state as numpy arrays, in the layout the CPU oracle dumps."""
         sc = self.scalars()

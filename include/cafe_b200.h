@@ -71,6 +71,8 @@ int cafe_sketch_tuning(void* handle, int window, int round_cap);
 /* out[13] = calls, lookups, rounds, jobs, truncated_jobs, resets, resets_refused, flips,
  * seq_fallbacks, main_hits, lru_visits, events, max_rounds */
 int cafe_sketch_stats(void* handle, int64_t* out13);
+/* How many of `jobs` ran in one launch each (the others took a launch per step). */
+int64_t cafe_sketch_one_launch_jobs(void* handle);
 /* Full state to / from host arrays ([4*n1], [n1], [4*n2], [n2], FIFO front to back).  No counterpart
  * in tricks/sketch.cpp (its state cannot be saved); layout follows save_state/load_state of
  * TOIS_revision/PinSAGE/sketch.cpp:333-402 in spirit. */

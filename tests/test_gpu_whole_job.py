@@ -29,7 +29,12 @@ def _run(step_by_step, lim, thr, alpha, calls, n, dom, fuse, unit, cap, seed):
     finally:
         profile.enable(False)
         profile.read()
-    return out, sk.state(), sk.stats()
+    return out, sk.state(), sk.stats(), sk.one_launch_jobs()
+
+
+# what a case is there for: it must have happened in the one-launch run
+REACHED = {(40, 96): ("resets", "flips"), (300, 33): ("truncated_jobs", "resets", "flips"), (300, 129): ("resets",),
+           (2000, 1024): ("truncated_jobs", "resets"), (20_000, 4096): ("resets",), (500, 700): ("truncated_jobs", "seq_fallbacks")}
 
 
 @pytest.mark.parametrize("lim,thr,alpha,calls,n,dom,fuse,unit,cap", [
@@ -48,6 +53,10 @@ def test_one_launch_equals_step_by_step(lim, thr, alpha, calls, n, dom, fuse, un
     from oracle.hotsketch import states_equal
     a = _run(True, lim, thr, alpha, calls, n, dom, fuse, unit, cap, n + lim)
     b = _run(False, lim, thr, alpha, calls, n, dom, fuse, unit, cap, n + lim)
+    assert a[3] == 0
+    assert b[3] == (b[2]["jobs"] if n * fuse <= 131_072 else 0) and b[2]["jobs"] > 0
+    for what in REACHED.get((lim, n), ()):
+        assert b[2][what] > 0, what
     for c, (u, v) in enumerate(zip(a[0], b[0])):
         assert u[2] == v[2], c
         assert np.array_equal(u[0], v[0]) and np.array_equal(u[1], v[1]), c
