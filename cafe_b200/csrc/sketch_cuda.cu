@@ -1518,6 +1518,13 @@ __global__ void __launch_bounds__(128) k_lru_pass_compact(const __grid_constant_
 // (the timeline's steps take one position or op per thread there: a chain of dependent loads each, so four or eight in a row
 // per thread, as in the launches of their own, took 6 to 19 us a step)
 #define CAFE_JOB_RESIDENT 3      // blocks per SM (the list replay takes 168 registers)
+// Three blocks take all registers of an SM, and a cooperative launch starts only when there is room for all its blocks at once.
+// With blocks for every SM, one block of anybody's on another stream held up the whole insert until it ended: a 6.6 ms
+// kernel of one block made an insert of 26 x 2048 lookups take 6.5 ms instead of 0.2; a collective waiting 300 us for its
+// peers made the backward beside it take 429 us instead of 348.  So a few SMs' worth of blocks is left out; blocks of others may
+// then fill as many SMs.  It costs nothing that can be seen: 26 x 2048 lookups into 108 000 buckets 180 us with and without,
+// into 360 000 buckets 211 (with 8 SMs left out 184 and 212).
+#define CAFE_JOB_SPARE_SMS 4
 // (the scratch of the timeline's blocks, tl_blk and tl_agg, is sized for blocks of CAFE_TL_SMALL)
 static_assert(CAFE_JOB_THREADS >= CAFE_TL_SMALL && CAFE_TL_BLOCK >= CAFE_TL_SMALL, "timeline blocks smaller than their scratch allows for");
 
@@ -1853,7 +1860,7 @@ struct CudaBackend {
     CafeJobOutcome* job_out = nullptr;    // what it reports, in host memory
     int32_t job_ticket = 0;
     int64_t jobs_launched = 0;            // jobs that went by it
-    int job_blocks = 0;                   // blocks of it that are resident at once (0: no cooperative launches here)
+    int job_blocks = 0;                   // most blocks of it (0: no cooperative launches here)
 
     ~CudaBackend() {
         if (cub_tmp) cudaFree(cub_tmp);
@@ -1979,7 +1986,7 @@ struct CudaBackend {
             check(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
             check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
             check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_whole_job, CAFE_JOB_THREADS, 0));
-            job_blocks = coop ? sms * per : 0;
+            job_blocks = coop && sms > CAFE_JOB_SPARE_SMS ? (sms - CAFE_JOB_SPARE_SMS) * per : 0;
         }
         hot_nb[0] = n1; hot_nb[1] = n2;
         check(cudaMalloc(&miss.pre, 4 * ((size_t)cap + 1)));

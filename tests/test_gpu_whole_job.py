@@ -63,3 +63,35 @@ def test_one_launch_equals_step_by_step(lim, thr, alpha, calls, n, dom, fuse, un
     assert states_equal(a[1], b[1]) == []
     keys = ("calls", "lookups", "resets", "flips", "seq_fallbacks", "main_hits", "lru_visits")   # (rounds may differ: passes race with withdrawals)
     assert {k: a[2][k] for k in keys} == {k: b[2][k] for k in keys}
+
+
+def test_another_streams_block_does_not_hold_up_the_insert():
+    """A job in one launch over more buckets than fill the GPU, while one block of another stream runs for milliseconds: the
+    insert does not wait for it (all blocks of a cooperative launch start together)."""
+    import torch
+    from cafe_b200 import HotSketch
+    F, B = 26, 2048
+    sk = HotSketch(120_171, 1, 1, 1.0000005, max_lookups=F * B)
+    off = [B * f for f in range(F + 1)]
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    batches = [((800_000 * torch.rand(F * B, device="cuda", generator=gen) ** 3).to(torch.int32) + 1,
+                torch.rand(F * B, device="cuda", generator=gen)) for _ in range(4)]
+    x, side = torch.ones(2, 1 << 23, device="cuda"), torch.cuda.Stream()
+    torch.cumsum(x, 1)                                   # two rows: one block walks them, 13 ms
+    for ids, imp in batches:
+        sk.insert(ids, imp, off)
+    torch.cuda.synchronize()
+    overtook = 0
+    for ids, imp in batches:
+        begun, ended = torch.cuda.Event(), torch.cuda.Event()
+        with torch.cuda.stream(side):
+            begun.record()
+            torch.cumsum(x, 1)
+            ended.record()
+        begun.synchronize()
+        sk.insert(ids, imp, off)
+        torch.cuda.current_stream().synchronize()
+        overtook += not ended.query()
+        torch.cuda.synchronize()
+    assert sk.one_launch_jobs() == sk.stats()["jobs"] > 0
+    assert overtook == len(batches)
