@@ -1512,9 +1512,19 @@ __global__ void __launch_bounds__(128) k_lru_pass_compact(const __grid_constant_
 // (146 000 buckets) 149 us.  Training steps against the launches: Kaggle shape 441 -> 363 us, Terabyte 510 -> 464, Avazu
 // 408 -> 346, 11 x 777 342 -> 313, four modules of 2048 1253 -> 1144.
 #define CAFE_JOB_THREADS 128
-// Beyond this many lookups the passes are bound by their work and want the launches' occupancy (24 warps per SM against 12
-// here, and a launch of their own for the long buckets); it is where the radix sort changes its form too.
-#define CAFE_JOB_MOST 131072     // most lookups of a job's call
+// Which calls.  Where the passes are bound by their work they want the launches' occupancy (24 warps per SM against 12 here,
+// and a launch of their own for the long buckets).  That is so
+// - beyond 131 072 lookups, where the radix sort changes its form too;
+// - over tables of more than a million buckets, all of which every round clears and scans.  Inserts of 3328 / 53 248 lookups, one
+//   launch against launches: 800 000 buckets 139 / 243 us against 155 / 258, a million 156 / 286 against 164 / 317, 1.2 million
+//   176 / 285 against 176 / 274, 1.6 million 212 / 333 against 197 / 308, 6.4 million 650 / 755 against 485 / 560;
+// - where a large call meets a small sketch, so that the replays of its LRU buckets are long: with lookups squared over LRU buckets
+//   at 2.4 million (26 624 over 300; 53 248 over 1200) 225 and 218 us against 260 and 249, at 3.4 (131 066 over 5000) 274 against
+//   312, or 317 against 306 with a heavier head, at 4.7 (53 248 over 600) 270 against 276 or 257 against 251, at 6.9 (91 000
+//   over 1200) 295 against 306 or 304 against 289, at 14 (131 066 over 1200) 352 against 336 and 413 against 367.
+#define CAFE_JOB_MOST 131072               // most lookups of a call
+#define CAFE_JOB_MOST_BUCKETS (1 << 20)    // most buckets of both tables
+#define CAFE_JOB_MOST_REPLAY (1 << 22)     // most lookups squared over LRU buckets
 // (the timeline's steps take one position or op per thread there: a chain of dependent loads each, so four or eight in a row
 // per thread, as in the launches of their own, took 6 to 19 us a step)
 #define CAFE_JOB_RESIDENT 3      // blocks per SM (the list replay takes 168 registers)
@@ -1851,7 +1861,12 @@ struct CudaBackend {
     float *gather_simp1 = nullptr, *gather_simp2 = nullptr;
     int32_t* count_of(int t) const { return hot_counts + 4 * hot_set + 2 * t; }
     // jobs of the last sorted call go by the whole-job launch
-    bool carries(int64_t M, int n2) const { return job_blocks > 0 && !cafe_prof_serialise() && M <= CAFE_JOB_MOST && M < 256 * (int64_t)n2; }
+    // (lookups that outnumber the LRU buckets 256 times go by the compacted lists, which only the launches have)
+    bool carries(int64_t M) const {
+        const int64_t n1 = hot_nb[0], n2 = hot_nb[1];
+        return job_blocks > 0 && !cafe_prof_serialise() && M <= CAFE_JOB_MOST && M < 256 * n2 && n1 + n2 <= CAFE_JOB_MOST_BUCKETS &&
+               M * M <= CAFE_JOB_MOST_REPLAY * n2;
+    }
     uint8_t* hot_flag[2] = {nullptr, nullptr};
     int hot_nb[2] = {0, 0};
     int cap = 0;
@@ -2056,7 +2071,7 @@ struct CudaBackend {
             check(cafe_radix_sort(batch, st));
             batch.count = 0;
             gather_imp = nullptr;
-            find_pending = carries(M, find[1].nb);
+            find_pending = carries(M);
             if (!find_pending) find_now(st);
         }
         if (aside) {
@@ -2127,12 +2142,11 @@ struct CudaBackend {
         pass_join();
         check_launch();
     }
-    // A job the resident grid can carry, rounds and commit in one launch; false: the engine takes the steps itself.  Lookups
-    // that outnumber the LRU buckets 256 times go by the compacted lists, which only the launches have.
+    // A job the resident grid can carry, rounds and commit in one launch; false: the engine takes the steps itself.
     bool run_job(const CafeJob& J0, uint8_t* const marks[2], uint32_t* ring, double refit_above, int real_n, bool adjust,
                  int round_cap, CafeJobOutcome* out) {
         sort_join(0);
-        if (!carries(J0.M, J0.n2)) {
+        if (!carries(J0.M)) {
             if (find_pending) {   // (timing was switched on since the sort)
                 find_now(stream);
                 if (gather_imp) gather_counts(gather_imp, J0.ord1, J0.ord2, J0.M, gather_simp1, gather_simp2);

@@ -48,13 +48,20 @@ REACHED = {(40, 96): ("resets", "flips"), (300, 33): ("truncated_jobs", "resets"
     (20_000, 1, 1.0000005, 3, 131_073, 200_000, 1, False, 0),
     (400_000, 1, 1.0000005, 4, 5000, 3_000_000, 20, False, 0),
     (500, 1, 1.0000005, 6, 700, 2000, 3, False, 1),
+    (60_000, 2, 1.0000005, 4, 131_072, 400_000, 1, False, 0),       # the largest call
+    (12_000, 1, 1.0000005, 4, 70_900, 300_000, 1, False, 0),        # just short of the largest call for 1200 LRU buckets
+    (12_000, 1, 1.0000005, 4, 71_000, 300_000, 1, False, 0),        # and just beyond
+    (1_048_576, 1, 1.0000005, 3, 2000, 3_000_000, 7, False, 0),     # two tables of 2^20 buckets less one
+    (1_048_590, 1, 1.0000005, 3, 2000, 3_000_000, 7, False, 0),     # and more than 2^20
 ])
 def test_one_launch_equals_step_by_step(lim, thr, alpha, calls, n, dom, fuse, unit, cap):
     from oracle.hotsketch import states_equal
     a = _run(True, lim, thr, alpha, calls, n, dom, fuse, unit, cap, n + lim)
     b = _run(False, lim, thr, alpha, calls, n, dom, fuse, unit, cap, n + lim)
     assert a[3] == 0
-    assert b[3] == (b[2]["jobs"] if n * fuse <= 131_072 else 0) and b[2]["jobs"] > 0
+    n1, n2 = int(lim * 0.9), int(lim * 0.1)
+    one = [m <= 131_072 and n1 + n2 <= 1 << 20 and m * m <= n2 << 22 and m < 256 * n2 for m in (u[0].size for u in b[0])]
+    assert b[3] == (b[2]["jobs"] if one[0] else 0) and b[2]["jobs"] > 0 and len(set(one)) == 1
     for what in REACHED.get((lim, n), ()):
         assert b[2][what] > 0, what
     for c, (u, v) in enumerate(zip(a[0], b[0])):
