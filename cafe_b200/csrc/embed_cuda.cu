@@ -668,8 +668,10 @@ __global__ void k_labels_to_float(const int32_t* __restrict__ label, int B, floa
 int cafe_embed_ws_init(CafeEmbedWorkspace* ws, int cap, int hotn) {
     ws->cap = cap;
     const size_t M = (size_t)cap;
+    // chunks of the largest call in either length (a call uses one of them)
     const size_t small = M < CAFE_CHUNK_SMALL_MOST ? M : CAFE_CHUNK_SMALL_MOST;
-    const size_t chunks = (M + CAFE_CHUNK - 1) / CAFE_CHUNK + (small + CAFE_CHUNK_SMALL - 1) / CAFE_CHUNK_SMALL;
+    const size_t short_chunks = (small + CAFE_CHUNK_SMALL - 1) / CAFE_CHUNK_SMALL, long_chunks = (M + CAFE_CHUNK - 1) / CAFE_CHUNK;
+    const size_t chunks = short_chunks > long_chunks ? short_chunks : long_chunks;
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t n) { if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1); };
     A((void**)&ws->norm, 4 * M); A((void**)&ws->imp, 4 * M); A((void**)&ws->totals, 4 * CAFE_MAX_SEGMENTS);
@@ -678,7 +680,7 @@ int cafe_embed_ws_init(CafeEmbedWorkspace* ws, int cap, int hotn) {
     A((void**)&ws->partial, sizeof(float) * 2 * chunks * CAFE_MAX_DIM);
     A((void**)&ws->row_winner, 4 * (size_t)(hotn > 0 ? hotn : 1));
     if (e == cudaSuccess) e = cudaMemset(ws->row_winner, 0xff, 4 * (size_t)(hotn > 0 ? hotn : 1));   // -1: unclaimed
-    A((void**)&ws->sort_scratch, 4 * cafe_rs_scratch_elems());
+    A((void**)&ws->sort_scratch, 4 * cafe_rs_scratch_elems(cap));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ws->late, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ws->ev_late, cudaEventDisableTiming);
     if (e != cudaSuccess) { cafe_internal_set_error(cudaGetErrorString(e)); return CAFE_ERR_CUDA; }

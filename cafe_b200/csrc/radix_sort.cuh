@@ -48,7 +48,7 @@ struct CafeSortDesc {
     uint2* tmp;              // [n] pairs between two passes
     uint2* out;              // [n] sorted (id or key, position)
     int32_t* start;          // [mod.n + 1] first sorted index whose key is >= k, or null
-    int32_t* scratch;        // cafe_rs_scratch_elems() int32: totals[digit], hist[block][digit]
+    int32_t* scratch;        // cafe_rs_scratch_elems(n) int32: totals[digit], hist[block][digit]
     int32_t passes, bits, blocks;
 };
 struct CafeSortBatch {
@@ -62,7 +62,13 @@ struct CafeSortShared {
     int32_t warp[CAFE_RS_WARPS];
 };
 
-static inline size_t cafe_rs_scratch_elems() { return (size_t)CAFE_RS_MAX_BINS * (CAFE_RS_MAX_BLOCKS + 1); }
+// blocks of a sort of n pairs in the launch-per-step form (a block ranks several tiles, one by one, where there are more)
+static inline int cafe_rs_blocks(int64_t n) {
+    const int64_t t = (n + CAFE_RS_TILE - 1) / CAFE_RS_TILE;
+    return (int)(t < CAFE_RS_MAX_BLOCKS ? t : CAFE_RS_MAX_BLOCKS);
+}
+// scratch of a sort of at most `cap` pairs
+static inline size_t cafe_rs_scratch_elems(int64_t cap) { return (size_t)CAFE_RS_MAX_BINS * (size_t)(cafe_rs_blocks(cap) + 1); }
 
 __device__ __forceinline__ uint32_t cafe_rs_key(const CafeSortDesc& D, uint32_t a) {
     return D.hashed == 1 ? (uint32_t)cafe_hash(a, D.mod) : D.hashed == 2 ? a % (uint32_t)D.mod.n : a;
@@ -405,8 +411,7 @@ static inline cudaError_t cafe_radix_sort(CafeSortBatch& B, cudaStream_t st) {
         return e != cudaSuccess ? e : g;
     }
     for (int s = 0; s < B.count; ++s) {
-        const int64_t t = ((int64_t)B.d[s].n + CAFE_RS_TILE - 1) / CAFE_RS_TILE;   // (a block ranks several tiles, one by one, where there are more)
-        B.d[s].blocks = (int)(t < CAFE_RS_MAX_BLOCKS ? t : CAFE_RS_MAX_BLOCKS);
+        B.d[s].blocks = cafe_rs_blocks(B.d[s].n);
         blocks = B.d[s].blocks > blocks ? B.d[s].blocks : blocks;
     }
     const dim3 grid((unsigned)blocks, (unsigned)B.count);

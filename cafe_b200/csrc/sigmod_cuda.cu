@@ -433,7 +433,7 @@ int cafe_sigmod_create(void** out, int lim, int threshold, double decay_rate, in
     auto A = [&](void** p, size_t n) { if (e == cudaSuccess) e = cudaMalloc(p, n ? n : 1); };
     A((void**)&H->b, sizeof(SgBucket) * (size_t)lim); A((void**)&H->ring, 4 * (size_t)rc); A((void**)&H->st, sizeof(SgState));
     A((void**)&H->ent, sizeof(uint2) * M); A((void**)&H->ent_tmp, sizeof(uint2) * M); A((void**)&H->start, 4 * ((size_t)lim + 1)); A((void**)&H->rank, 4 * M);
-    A((void**)&H->blk, 4 * nblk); A((void**)&H->sort_scratch, 4 * cafe_rs_scratch_elems()); A((void**)&H->simp, 4 * M);
+    A((void**)&H->blk, 4 * nblk); A((void**)&H->sort_scratch, 4 * cafe_rs_scratch_elems(max_lookups)); A((void**)&H->simp, 4 * M);
     A((void**)&H->cand, M > (size_t)lim + 1 ? M : (size_t)lim + 1); A((void**)&H->partial, 8 * nblk);
     if (e == cudaSuccess) e = cudaMemset(H->b, 0, sizeof(SgBucket) * (size_t)lim);
     if (e == cudaSuccess) {

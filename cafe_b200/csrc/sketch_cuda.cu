@@ -1981,7 +1981,7 @@ struct CudaBackend {
         batch.count = 0;
         for (int i = 0; i < 2; ++i) {
             check(cudaMalloc(&sort_tmp[i], sizeof(uint2) * (size_t)cap));
-            check(cudaMalloc(&sort_scratch[i], 4 * cafe_rs_scratch_elems()));
+            check(cudaMalloc(&sort_scratch[i], 4 * cafe_rs_scratch_elems(cap)));
         }
         // (highest priority: the sorts are chains of small steps that run beside streaming kernels filling every SM;
         // their blocks must not queue behind those)

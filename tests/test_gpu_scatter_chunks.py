@@ -47,3 +47,19 @@ def test_sums_of_rows_of_every_length(n, kind, D):
     want_h.index_add_(0, -row[is_hot].long(), -grad[is_hot])
     want_c.index_add_(0, row[~is_hot].long(), -grad[~is_hot])
     assert torch.equal(high, want_h) and torch.equal(cold, want_c)
+
+
+def test_small_handles_hold_little_memory():
+    """Workspaces are sized for the calls a handle was made for: sketches of 1000 rows and 2048 lookups, whose arrays add up to
+    about 1 MB (one-stage: 0.2 MB), take no more than one of the driver's granules of 2 MiB each (one-stage sketches share them)."""
+    import torch
+    from cafe_b200 import HotSketch
+    from cafe_b200.sigmod import SigmodSketch
+    for make, granules in ((lambda: HotSketch(1000, max_lookups=2048), 32), (lambda: SigmodSketch(1000, 1, max_lookups=2048), 8)):
+        first = make()
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        held = [make() for _ in range(32)]
+        torch.cuda.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] <= granules * 2**21
+        del held, first
