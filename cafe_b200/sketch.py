@@ -19,9 +19,16 @@ _STATE_ARRAYS = ["main_val", "main_cnt", "main_dic", "main_flip", "lru_val", "lr
                  "lru_flip", "queue"]
 
 
+# torch's own accessor for launchers makes no Stream object (0.3 us a call against 3.3), but it is not public:
+# a torch without it gets the public form
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    """The current device's current stream as a raw handle (torch's own accessor for launchers: no Stream object is made)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    """The current device's current stream as a raw handle."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _np_ptr(a: np.ndarray, typ):

@@ -203,3 +203,16 @@ def test_random_configurations(block):
         n = int(r.integers(200, 6000)); dom = int(r.choice([30, 200, 3000, 200000])); fuse = int(r.integers(1, 8))
         drive(lim, thr, alpha, fuse * 6, n, dom, fuse, seed=1000 + seed, zero_ids=seed % 3 == 0, ragged=seed % 4 == 1,
               unit=seed % 5 == 2)
+
+
+def test_stream_handle_with_and_without_the_private_accessor(monkeypatch):
+    """The launching stream is the current one, on the default stream and on others, also where torch has no private accessor."""
+    import torch
+    from cafe_b200 import sketch
+    side = torch.cuda.Stream()
+    for private in (True, False):
+        if not private:
+            monkeypatch.setattr(sketch, "_raw_stream", None)
+        assert sketch._stream() == torch.cuda.current_stream().cuda_stream
+        with torch.cuda.stream(side):
+            assert sketch._stream() == side.cuda_stream
