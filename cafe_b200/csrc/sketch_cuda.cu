@@ -1966,10 +1966,6 @@ struct CudaBackend {
             check_launch();
             await(ticket, want);
             memcpy(d, pinned, n);
-        } else if (pinned && n <= 4092) {
-            check(cudaMemcpyAsync(pinned, s, n, cudaMemcpyDeviceToHost, stream));
-            check(cudaStreamSynchronize(stream));
-            memcpy(d, pinned, n);
         } else {
             check(cudaMemcpyAsync(d, s, n, cudaMemcpyDeviceToHost, stream));
             check(cudaStreamSynchronize(stream));
@@ -2095,7 +2091,8 @@ struct CudaBackend {
         k_gather_counts<<<cafe_blocks(M), CAFE_TPB, 0, stream>>>(imp, ord1, ord2, M, simp1, simp2);
         check_launch();
     }
-    // makes `stream` wait for the sorts outstanding on the side stream (no-op when there are none)
+    // makes `stream` wait for the sorts outstanding on the side stream (no-op when there are none; one batch makes both orders,
+    // so it does not matter which of them is asked for)
     void sort_join(int) {
         if (!side_pending) return;
         check(cudaStreamWaitEvent(stream, ev_join, 0));
