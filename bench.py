@@ -632,7 +632,8 @@ def run_ours(args, rank, world, local_rank):
                 "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                         "ms_per_step": ms_e2e / K},
                 "gpu_launches": int(launches), "clocks": clocks, "roofline": roof, "sketch_mix": mix, "phases": phases,
-                "phases_note": "per-kernel CUDA-event times of a separate pass with the side-stream overlap switched off",
+                "phases_note": "per-kernel CUDA-event times of a separate pass with the side-stream overlap switched off and a "
+                               "launch per step of every insert job (calls of up to 131 072 lookups otherwise take one launch)",
                 "ms_per_step_profiled": ms_prof / K}
         if rank_info is not None:
             line["ranks"] = rank_info

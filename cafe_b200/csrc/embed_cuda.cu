@@ -904,7 +904,7 @@ int cafe_grad_importance(void* h, const float* grad_dev, int64_t field_stride, i
 // workspace that cafe_sketch_create obtained with cudaMalloc.  Some hosts cannot do that: a serving
 // process that handed the whole device to its own memory pool at start-up and forbids further
 // allocation, or a caller that must not take the device-wide stall an allocation can cause in the
-// middle of its step.  For them the same three kernels run here on a scratch area that is part of
+// middle of its step.  For them the same kernels run here on a scratch area that is part of
 // the library image: a file-scope __device__ array, which every GPU that loads the library holds
 // from load to exit (CAFE_STATIC_IMPORTANCE_MAX floats for the norms plus one float per field,
 // about 1 MiB).  No handle is needed, and nothing is allocated or freed here: not with the CUDA
@@ -983,8 +983,8 @@ int cafe_migrate(void* h, const void* ids_dev, int ids_are_int64, const int32_t*
 }
 
 // The scatter in two parts.  scatter_prepare needs only the forward's row numbers (unified row keys and
-// their radix sort); scatter_apply reads the sorted keys, the gradient and the tables.  The split lets a
-// caller run the first part on the workspace's side stream while the sketch insert runs on the main one.
+// their radix sort); scatter_apply reads the sorted keys, the gradient and the tables.  Backward calls with a parallel insert
+// have the first part done in one batch with the insert's own sorts (start_sorts).
 static CafeSortDesc row_sort_desc(CafeEmbedWorkspace* ws, const CafeFields& F, int total) {
     // (row key, position) pairs, stable: a row's lookups stay in batch order, which fixes the order of the additions
     CafeSortDesc D;
@@ -1087,7 +1087,7 @@ static int backward_side_work(void* h, CafeEmbedWorkspace* ws, const CafeFields&
 // The whole post-backward part of one training step for `nfields` fields, in the reference's order:
 // importance -> sketch insert (one call per field, ascending) -> migration with pre-update rows ->
 // SGD with the forward-time rows.
-// importance of the fields [f0, f0 + nf) of a call over `nfields` fields: the same three kernels as
+// importance of the fields [f0, f0 + nf) of a call over `nfields` fields: the same kernels as
 // cafe_grad_importance, on that range of the workspace
 static int importance_range(CafeEmbedWorkspace* ws, const float* grad_dev, int64_t field_stride, int64_t sample_stride, int f0,
                             int nf, int B, int D, float* imp_dev, cudaStream_t st) {

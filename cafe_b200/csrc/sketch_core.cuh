@@ -47,7 +47,7 @@ CAFE_HD int32_t cafe_hash(uint32_t x, int32_t n) {
 
 // The same remainder by a divisor that is known ahead: q = high word of v * floor(2^64 / n) is the quotient or one less
 // (v < 2^62), so one conditional subtraction ends it.  A dozen instructions instead of the hundred of a 64-bit
-// division; every kernel that hashes ids takes it.
+// division; every kernel that hashes many ids takes it (the sequential insert, one thread after another, divides).
 struct CafeMod { uint64_t magic; int32_t n; };
 static inline CafeMod cafe_mod_of(int32_t n) {
     CafeMod m;

@@ -1504,8 +1504,9 @@ __global__ void __launch_bounds__(128) k_lru_pass_compact(const __grid_constant_
 // A round is eight or nine steps of microseconds each, and a job has three to six rounds.  Launched one by one with a
 // read-back per round they are nearly all launch gaps and waits of the host.  So jobs that a resident grid can carry run
 // in ONE cooperative launch: the steps are separated by the grid's barrier, every block takes the round's decision (go on,
-// shorten the job at a re-fit, finish) from the round result itself, and the host reads one record at the end.  The
-// steps are the functions of the launches above; the job lives in shared memory because rounds and shortenings change it.
+// shorten the job at a re-fit, finish) from the round result itself, and the host reads one record, written as soon as the
+// rounds have converged: the final pass and the commit follow it, and what the host queues next follows them.  The steps
+// are the functions of the launches above; the job lives in shared memory because rounds and shortenings change it.
 //
 // What bounds it is the chain of dependent loads of every step and the slowest bucket of a pass; a barrier takes 1.2 us.  A
 // step's insert of 26 x 128 lookups (12 000 buckets) takes 91 us of it, of 26 x 2048 (108 000 buckets) 147 us, of 9 x 4096

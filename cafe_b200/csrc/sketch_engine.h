@@ -151,7 +151,7 @@ public:
         return be.ok() ? CAFE_OK : CAFE_ERR_CUDA;
     }
 
-    // Starts the bucket sorts of the next insert_segments call early, on the backend's side lanes, for
+    // Starts the bucket sorts of the next insert_segments call early, on the backend's side lane, for
     // a caller that knows the ids before it knows the counts.  Only honoured when that call passes the
     // same pointer and its whole input is one stretch of n lookups.  The sorts read `ids`, which holds
     // the same values in memory that outlives them.

@@ -1,4 +1,8 @@
-"""Per-kernel timing of the library's own launches (CUDA events on the launching stream) and launch counts."""
+"""Per-kernel timing of the library's own launches (CUDA events on the launching stream) and launch counts.
+
+While timing is on, every kernel runs alone on the caller's stream and every job of an insert takes a launch per step.  Calls of
+up to 131 072 lookups otherwise run a job in one launch, so the figures of such calls are those of launches that a step
+without timing does not make."""
 from __future__ import annotations
 
 import ctypes

@@ -173,7 +173,7 @@ class _PeerFunction(torch.autograd.Function):
             wp, hp = f.ptrs()
             out_rank = pb.ptr_array(pb.h_pooled, pb.block_off[plan.rank], 4)
             if training:
-                # sketch probe, then the backward's sorts on the side streams, then the gather with the exchange as
+                # sketch probe, then the backward's sorts on the side stream, then the gather with the exchange as
                 # its epilogue: the sorts run beside the gather and the dense model
                 f.resolve_begin(own, gid, row, grp.insert_mode)
                 _lib.check(lib.cafe_embed_gather_sharded(grp.sketch.handle, row.data_ptr(), Fg, G * Bl, f.hash_size, wp, hp,

@@ -96,7 +96,7 @@ class _FieldSet:
 
     def forward_training(self, ids: torch.Tensor, out: torch.Tensor, field_stride: int, sample_stride: int, mode: int):
         """forward() in two kernels with the backward's head start in between: the sketch probe first, then the
-        bucket sorts of the insert and the row sort of the scatter are started on the library's side streams, and
+        bucket sorts of the insert and the row sort of the scatter are started on the library's side stream, and
         the row gather runs beside them.  Same results as forward()."""
         lib, sk = self.sketch.lib, self.sketch
         B = ids.numel() // self.nf

@@ -300,7 +300,9 @@ int cafe_global_set_capacity(int max_len);
 
 /* ---- measurement ---------------------------------------------------------------------------------
  * No counterpart in the reference.  Kernel launches of the library are always counted per slot;
- * with cafe_profile_enable(1) each launch is also bracketed by CUDA events on its stream.
+ * with cafe_profile_enable(1) each launch is also bracketed by CUDA events on its stream, nothing runs
+ * beside it, and every insert job takes a launch per step (calls of up to 131 072 lookups otherwise run a
+ * job in one launch, so their figures are those of launches that an untimed step does not make).
  * cafe_profile_read fills ms[slots] (event time summed per slot) and launches[slots] since the last
  * read, after synchronising the device. */
 int cafe_profile_slots(void);

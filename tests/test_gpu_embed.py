@@ -371,11 +371,11 @@ def test_a_dropped_forward_leaves_nothing_behind():
             np.testing.assert_allclose(grp.weight_hash[f].detach().cpu().numpy(), orc.wc[f], rtol=1e-5, atol=1e-7)
 
 
-@pytest.mark.parametrize("B", [20_000, 70_000])
+@pytest.mark.parametrize("B", [300, 20_000, 70_000])
 def test_a_dropped_forwards_sorts_survive_its_buffers(B):
     """The head start of a forward whose backward never comes is still sorting when its id and row arrays are written again, by
-    the next forward or by whatever got their memory.  In the forms of the sort that read their keys twice (several tiles per
-    block of a cluster, a launch per step), at a call as large as the workspace.  The next batch's step must be that of a
+    the next forward or by whatever got their memory.  In every form of the sort (at most a tile per block, several tiles per
+    block of a cluster, a launch per step; the last two read their keys twice), at a call as large as the workspace.  The next batch's step must be that of a
     group which never dropped a forward and inserts one lookup at a time."""
     import torch
     import cafe_b200

@@ -1,5 +1,5 @@
-"""The one-launch radix sort where every block has at most a tile of pairs (pairs kept in shared memory by a block that sorts
-alone, histograms exchanged in a cluster otherwise), around the sizes where the number of blocks or the form changes; keys of
+"""The one-launch radix sort where every block has at most a tile of pairs (read once per pass and ranked without a histogram
+step; the blocks of a cluster exchange their counts), around the sizes where the number of blocks or the form changes; keys of
 one, two and three passes.  Same checks as the sort's other sizes: exact scatter sums, and the sequential insert's state."""
 import pytest
 
