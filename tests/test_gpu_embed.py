@@ -336,8 +336,8 @@ def test_two_fields_claim_one_hot_row_in_one_step():
 
 def test_a_dropped_forward_leaves_nothing_behind():
     """A training forward whose backward never comes (its head start is under way, its buffers are freed), then a forward
-    in eval mode whose buffers the allocator places at the same addresses, and that one's backward: the row order and the
-    bucket orders must be those of the second batch."""
+    in eval mode whose buffers the allocator may place at the same addresses (the next test makes sure of it), and that one's
+    backward: the row order and the bucket orders must be those of the second batch."""
     import torch
     import cafe_b200
     from oracle.hotsketch import OracleSketch, states_equal
